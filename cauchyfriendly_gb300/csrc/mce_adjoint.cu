@@ -478,15 +478,16 @@ __device__ inline DD dneg(DD a) { return DD{-a.v, -a.t}; }
 __device__ inline DD dmul(DD a, DD b) { return DD{a.v * b.v, a.t * b.v + a.v * b.t}; }
 __device__ inline DD ddiv(DD a, DD b)
 {
-    const double q = a.v / b.v;
-    return DD{q, (a.t - q * b.t) / b.v};
+    const mce::DivBy by = mce::div_by(b.v);
+    const double q = mce::divide(a.v, by);
+    return DD{q, mce::divide(a.t - q * b.t, by)};
 }
-// a / b with rb = 1 / b.v: the value divides (the same double as the
-// forward run), the tangent multiplies by the shared reciprocal (a row
-// normalised by one norm divides d values by it)
-__device__ inline DD ddiv_r(DD a, DD b, double rb)
+// a / b with rb = 1 / b.v, by = div_by(b.v): the value divides (the same
+// double as the forward run), the tangent multiplies by the shared reciprocal
+// (a row normalised by one norm divides d values by it)
+__device__ inline DD ddiv_r(DD a, DD b, const mce::DivBy& by, double rb)
 {
-    const double q = a.v / b.v;
+    const double q = mce::divide(a.v, by);
     return DD{q, (a.t - q * b.t) * rb};
 }
 __device__ inline DD dabs(DD x) { return x.v < 0 ? dneg(x) : (x.v > 0 ? x : DD{0.0, 0.0}); }
@@ -564,8 +565,9 @@ __global__ void __launch_bounds__(128) k_adj_chain(ChainArgs a)
         for (int i = 0; i < pncc; i++) {
             DD nf = dd(0.0);
             for (int j = 0; j < d; j++) nf = dadd(nf, dabs(Gt[i * d + j]));
-            const double rnf = 1.0 / nf.v;
-            for (int j = 0; j < d; j++) Gt[i * d + j] = ddiv_r(Gt[i * d + j], nf, rnf);
+            const mce::DivBy by = mce::div_by(nf.v);
+            const double rnf = mce::divide(1.0, by);
+            for (int j = 0; j < d; j++) Gt[i * d + j] = ddiv_r(Gt[i * d + j], nf, by, rnf);
             bt[i] = dmul(bt[i], nf);
         }
         bool F[kGammaMax];
@@ -612,8 +614,9 @@ __global__ void __launch_bounds__(128) k_adj_chain(ChainArgs a)
             DD n1 = dd(0.0);
             for (int j = 0; j < d; j++) n1 = dadd(n1, dabs(A[i * d + j]));
             P[i] = dmul(P[i], n1);
-            const double rn1 = 1.0 / n1.v;
-            for (int j = 0; j < d; j++) A[i * d + j] = ddiv_r(A[i * d + j], n1, rn1);
+            const mce::DivBy by = mce::div_by(n1.v);
+            const double rn1 = mce::divide(1.0, by);
+            for (int j = 0; j < d; j++) A[i * d + j] = ddiv_r(A[i * d + j], n1, by, rn1);
         }
         bool Fg[kGammaMax];
         for (int j = 0; j < cnt; j++) Fg[j] = true;
@@ -695,8 +698,9 @@ __global__ void __launch_bounds__(128) k_adj_chain(ChainArgs a)
                 DD n1 = dd(0.0);
                 for (int j = 0; j < d; j++) n1 = dadd(n1, dabs(cA[i * d + j]));
                 cp[i] = dmul(cp[i], n1);
-                const double rn1 = 1.0 / n1.v;
-                for (int j = 0; j < d; j++) cA[i * d + j] = ddiv_r(cA[i * d + j], n1, rn1);
+                const mce::DivBy by = mce::div_by(n1.v);
+                const double rn1 = mce::divide(1.0, by);
+                for (int j = 0; j < d; j++) cA[i * d + j] = ddiv_r(cA[i * d + j], n1, by, rn1);
             }
             if (tt != m) {
                 bool F[MR], hflag[MR];

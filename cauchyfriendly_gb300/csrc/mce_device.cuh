@@ -9,6 +9,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "mce_div.cuh"
+
 namespace mce {
 
 constexpr int kMaxRows = 31;    // keys are 32-bit sign masks (cauchy_estimator.hpp:231-235)
@@ -60,18 +62,19 @@ __device__ inline unsigned long long dabs_bits(double x);
 // den = d r + c, (b r + a)/den, (b - a r)/den; |c| < |d|: r = c/d,
 // den = c r + d, (a r + b)/den, (b r - a)/den), so the results are the same
 // bits and lanes of a warp that would take different branches no longer
-// execute both.
+// execute both.  The three divisions run on the integer pipe (mce_div.cuh).
 __device__ inline cd cdiv(cd x, cd y)
 {
     const double a = x.re, b = x.im, c = y.re, d = y.im;
     const bool big_c = !(dabs_bits(c) < dabs_bits(d));
     const double p = big_c ? c : d, q = big_c ? d : c;
     const double P = big_c ? a : b, Q = big_c ? b : a;
-    const double r = q / p;
+    const double r = divide(q, p);
     const double den = q * r + p;
     const double pr = P * r;
     const double num = big_c ? (Q - pr) : (pr - Q);
-    return cd{(Q * r + P) / den, num / den};
+    const DivBy by = div_by(den);
+    return cd{divide(Q * r + P, by), divide(num, by)};
 }
 
 // Comparisons of doubles on their bit patterns (integer pipe).  IEEE doubles
@@ -219,50 +222,57 @@ __device__ inline int orientation_mask(const double* Ai, const double* Aj, int m
 // ---------------------------------------------------------------------------
 // Dense D x D linear algebra in the reference's operation order
 // (cauchy_linalg.hpp:1180-1390).
+// Every index is a compile-time one (row exchanges are selects), so the
+// matrix stays in registers.  The exchanges are applied to b as well, and
+// perm[i] receives the row of the matrix that ends at row i.  piv receives
+// the divisors of the U factor's diagonal: the elimination divides by the
+// first D - 1 of them, every solve by all D.
 template <int D>
-__device__ inline bool plu(double* A, int* P)
+__device__ inline bool plu(double* A, double* b, int* perm, DivBy* piv)
 {
+#pragma unroll
+    for (int i = 0; i < D; i++) perm[i] = i;
+#pragma unroll
     for (int j = 0; j < D; j++) {
-        double piv = kPluEps;
+        double big = kPluEps;
         int pi = -1;
+#pragma unroll
         for (int i = j; i < D; i++)
-            if (abs_gt(A[i * D + j], piv)) {
-                piv = A[i * D + j];
+            if (abs_gt(A[i * D + j], big)) {
+                big = A[i * D + j];
                 pi = i;
             }
         if (pi == -1) return false;
-        if (pi != j)
+#pragma unroll
+        for (int i = j + 1; i < D; i++) {
+            const bool sw = pi == i;
+#pragma unroll
             for (int c = 0; c < D; c++) {
-                const double t = A[j * D + c];
-                A[j * D + c] = A[pi * D + c];
-                A[pi * D + c] = t;
+                const double t = A[j * D + c], u = A[i * D + c];
+                A[j * D + c] = sw ? u : t;
+                A[i * D + c] = sw ? t : u;
             }
-        P[j] = pi;
+            const double bj = b[j], bi = b[i];
+            b[j] = sw ? bi : bj;
+            b[i] = sw ? bj : bi;
+            const int pj = perm[j], pk = perm[i];
+            perm[j] = sw ? pk : pj;
+            perm[i] = sw ? pj : pk;
+        }
+        piv[j] = div_by(A[j * D + j]);
+#pragma unroll
         for (int k = j + 1; k < D; k++) {
-            A[k * D + j] /= A[j * D + j];
-            const double t = A[k * D + j];
+            const double t = divide(A[k * D + j], piv[j]);
+            A[k * D + j] = t;
+#pragma unroll
             for (int q = j + 1; q < D; q++) A[k * D + q] -= t * A[j * D + q];
         }
     }
     return true;
 }
 
-// Row permutation applied by the pivot list, inverted (cauchy_linalg.hpp:1258-1277).
 template <int D>
-__device__ inline void inverse_perm(const int* P, int* PT)
-{
-    int Preg[D];
-    for (int i = 0; i < D; i++) Preg[i] = i;
-    for (int i = 0; i < D; i++) {
-        const int t = Preg[i];
-        Preg[i] = Preg[P[i]];
-        Preg[P[i]] = t;
-    }
-    for (int i = 0; i < D; i++) PT[Preg[i]] = i;
-}
-
-template <int D>
-__device__ inline void lu_solve_inplace(const double* LU, double* x)
+__device__ inline void lu_solve_inplace(const double* LU, const DivBy* piv, double* x)
 {
 #pragma unroll
     for (int i = 0; i < D; i++) {
@@ -276,12 +286,9 @@ __device__ inline void lu_solve_inplace(const double* LU, double* x)
         double s = x[i];
 #pragma unroll
         for (int j = D - 1; j > i; j--) s -= LU[i * D + j] * x[j];
-        x[i] = s / LU[i * D + i];
+        x[i] = divide(s, piv[i]);
     }
 }
-
-template <int D>
-__device__ inline double cond1_from_lu(const double* A, const int* P, double nrm);
 
 // Upper bound on the 1-norm of (LU)^-1 from packed factors with partial
 // pivoting: ||A^-1|| <= ||M(U)^-1|| ||L^-1|| with M(U) the comparison matrix
@@ -313,64 +320,25 @@ __device__ inline float inv_norm1_bound(const double* LU)
     return best * (float)(1 << (D - 1)) * 1.0001f;
 }
 
-// 1-norm condition number through the explicit inverse; on success A holds
-// the packed LU factors and P the pivots.  Returns DBL_MAX when PLU fails.
+// cond(A) > eps for the 1-norm condition number through the explicit inverse
+// (cauchy_linalg.hpp:1369-1389: the 1-norm of A times the largest 1-norm of
+// an inverse column), from the packed LU factors: stops at the first inverse
+// column whose 1-norm s already gives nrm * s > eps: the full value is nrm
+// times the largest column norm, and rounding is monotone, so that column
+// settles the comparison exactly as the full computation would (the columns
+// are solved in the same order and the same arithmetic).  Nearly singular
+// subsets, whose every inverse column is large, then cost one solve instead
+// of D.
 template <int D>
-__device__ inline double cond1(double* A, int* P)
+__device__ inline bool cond1_exceeds(const double* LU, const DivBy* piv, const int* perm, double nrm, double eps)
 {
-    double nrm = -1;
-#pragma unroll
-    for (int c = 0; c < D; c++) {
-        double s = 0;
-#pragma unroll
-        for (int r = 0; r < D; r++) s += fabs(A[r * D + c]);
-        if (dlt(nrm, s)) nrm = s;
-    }
-    if (!plu<D>(A, P)) return 1.79769313486231570815e+308;
-    return cond1_from_lu<D>(A, P, nrm);
-}
-
-// The second half of cond1: 1-norm of the explicit inverse from the packed LU
-// factors, times the 1-norm of A (cauchy_linalg.hpp:1369-1389).
-template <int D>
-__device__ inline double cond1_from_lu(const double* A, const int* P, double nrm)
-{
-    int PT[D];
-    inverse_perm<D>(P, PT);
-    double inrm = -1;
-    (void)A;
-#pragma unroll
-    for (int i = 0; i < D; i++) {
-        double w[D];
-#pragma unroll
-        for (int j = 0; j < D; j++) w[j] = (j == PT[i]) ? 1.0 : 0.0;
-        lu_solve_inplace<D>(A, w);
-        double s = 0;
-#pragma unroll
-        for (int j = 0; j < D; j++) s += fabs(w[j]);
-        if (dlt(inrm, s)) inrm = s;
-    }
-    return nrm * inrm;
-}
-
-// cond1_from_lu(A, P, nrm) > eps, stopping at the first inverse column whose
-// 1-norm s already gives nrm * s > eps: the full value is nrm times the
-// largest column norm, and rounding is monotone, so that column settles the
-// comparison exactly as the full computation would (the columns are solved
-// in the same order and the same arithmetic).  Nearly singular subsets,
-// whose every inverse column is large, then cost one solve instead of D.
-template <int D>
-__device__ inline bool cond1_exceeds(const double* A, const int* P, double nrm, double eps)
-{
-    int PT[D];
-    inverse_perm<D>(P, PT);
     double inrm = -1;
 #pragma unroll
     for (int i = 0; i < D; i++) {
         double w[D];
 #pragma unroll
-        for (int j = 0; j < D; j++) w[j] = (j == PT[i]) ? 1.0 : 0.0;
-        lu_solve_inplace<D>(A, w);
+        for (int j = 0; j < D; j++) w[j] = (perm[j] == i) ? 1.0 : 0.0;
+        lu_solve_inplace<D>(LU, piv, w);
         double s = 0;
 #pragma unroll
         for (int j = 0; j < D; j++) s += fabs(w[j]);
@@ -378,15 +346,6 @@ __device__ inline bool cond1_exceeds(const double* A, const int* P, double nrm, 
         if (dlt(inrm, s)) inrm = s;
     }
     return nrm * inrm > eps;
-}
-
-template <int D>
-__device__ inline void solve_lu(const double* LU, const int* P, const double* b, double* x)
-{
-    int PT[D];
-    inverse_perm<D>(P, PT);
-    for (int i = 0; i < D; i++) x[PT[i]] = b[i];
-    lu_solve_inplace<D>(LU, x);
 }
 
 // ---------------------------------------------------------------------------

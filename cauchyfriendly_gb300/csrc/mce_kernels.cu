@@ -396,7 +396,7 @@ __global__ void k_first_build(const double* A0, const double* p0, const double* 
             rho[l] = p[l];
             Fi[l] = false;
         } else {
-            const double r = 1.0 / h;
+            const double r = divide(1.0, h);
             for (int j = 0; j < D; j++) mu[l * D + j] = A[l * D + j] * r;
             rho[l] = p[l] * ah;
             Fi[l] = true;
@@ -536,7 +536,8 @@ __global__ void k_tp(ParentList P, long long nP, const EstStep<D>* st, int with_
                 double n1 = 0;
                 for (int j = 0; j < D; j++) n1 += fabs(v[j]);
                 p[r] *= n1;
-                for (int j = 0; j < D; j++) A[r * D + j] = v[j] / n1;
+                const DivBy by = div_by(n1);
+                for (int j = 0; j < D; j++) A[r * D + j] = divide(v[j], by);
             }
             double wb[D];
             for (int j = 0; j < D; j++) wb[j] = b[j];
@@ -619,11 +620,12 @@ __global__ void k_build_B_vertices(ParentList P, long long nP, const long long* 
         const double* As = P.A + i * MC * D;
         const double* bp = bpert_all + (long long)P.est[i] * MC;
         const unsigned char* c = combos + combo_off[m] + (x - voff[i]) * D;
-        double Ac[D * D], bc[D], v[D];
-        int Pv[D];
+        double Ac[D * D], v[D];
+        int perm[D];
+        DivBy piv[D];
         for (int j = 0; j < D; j++) {
             for (int l = 0; l < D; l++) Ac[j * D + l] = As[c[j] * D + l];
-            bc[j] = bp[c[j]];
+            v[j] = bp[c[j]];
         }
         int out = -1;
         // cond(A) > 1e12 skips the vertex.  A single-precision upper bound from
@@ -636,10 +638,10 @@ __global__ void k_build_B_vertices(ParentList P, long long nP, const long long* 
             for (int r = 0; r < D; r++) sm += fabs(Ac[r * D + cc]);
             if (dlt(nrm, sm)) nrm = sm;
         }
-        if (plu<D>(Ac, Pv)) {
+        if (plu<D>(Ac, v, perm, piv)) {
             const double bound = nrm * (double)inv_norm1_bound<D>(Ac);
-            if ((bound <= 0.1 * kCondEps) || !cond1_exceeds<D>(Ac, Pv, nrm, kCondEps)) {
-                solve_lu<D>(Ac, Pv, bc, v);
+            if ((bound <= 0.1 * kCondEps) || !cond1_exceeds<D>(Ac, piv, perm, nrm, kCondEps)) {
+                lu_solve_inplace<D>(Ac, piv, v);
                 unsigned inmask = 0;
                 for (int j = 0; j < D; j++) inmask |= 1u << c[j];
                 int niv = 0;
@@ -884,7 +886,7 @@ __global__ void k_mu_rows(ParentList P, long long nP, const EstStep<D>* st, int*
                 for (int j = 0; j < D; j++) mu[l * D + j] = A[l * D + j];
                 rho[l] = p[l];
             } else {
-                const double r = 1.0 / h;
+                const double r = divide(1.0, h);
                 for (int j = 0; j < D; j++) mu[l * D + j] = A[l * D + j] * r;
                 rho[l] = p[l] * ah;
                 integ |= 1u << l;
@@ -1058,7 +1060,8 @@ __global__ void __launch_bounds__(128) k_mu_terms(ParentList P, long long nP, co
             double n1 = 0;
             for (int j = 0; j < D; j++) n1 += fabs(At[r * D + j]);
             pt[r] *= n1;
-            for (int j = 0; j < D; j++) At[r * D + j] /= n1;
+            const DivBy by = div_by(n1);
+            for (int j = 0; j < D; j++) At[r * D + j] = divide(At[r * D + j], by);
         }
         if (t != m) {
             mfin = mu_coalign_smem<D>(At, pt, qt, m, hof, R.cmap + slot * MC, R.csmap + slot * MC, err);
@@ -3065,8 +3068,9 @@ __global__ void k_cpdf2d_terms(ParentList P, long long a, long long n, int i1, i
                 continue;
             }
             const double s = f0 + f1;
-            A[2 * r] /= s;
-            A[2 * r + 1] /= s;
+            const DivBy by = div_by(s);
+            A[2 * r] = divide(A[2 * r], by);
+            A[2 * r + 1] = divide(A[2 * r + 1], by);
             p[r] *= s;
         }
         int mn = 0;
@@ -3111,9 +3115,9 @@ __global__ void k_cpdf2d_terms(ParentList P, long long a, long long n, int i1, i
             double pt0, pt1;
             if (fabs(a0) < fabs(a1)) {
                 pt0 = 1;
-                pt1 = -a0 / a1;
+                pt1 = divide(-a0, a1);
             } else {
-                pt0 = -a1 / a0;
+                pt0 = divide(-a1, a0);
                 pt1 = 1;
             }
             double t1 = atan2(pt1, pt0);
@@ -3273,8 +3277,9 @@ __global__ void __launch_bounds__(128) k_rel2d_pairs(Rel2DArgs a)
             }
             F |= 1u << i;
             const double s = f0 + f1;
-            A2[2 * i] /= s;
-            A2[2 * i + 1] /= s;
+            const DivBy by = div_by(s);
+            A2[2 * i] = divide(A2[2 * i], by);
+            A2[2 * i + 1] = divide(A2[2 * i + 1], by);
             pr[i] *= s;
         }
         int mn = 0;
@@ -3361,9 +3366,9 @@ __global__ void __launch_bounds__(128) k_rel2d_pairs(Rel2DArgs a)
             double pt0, pt1;
             if (fabs(a0) < fabs(a1)) {
                 pt0 = 1;
-                pt1 = -a0 / a1;
+                pt1 = divide(-a0, a1);
             } else {
-                pt0 = -a1 / a0;
+                pt0 = divide(-a1, a0);
                 pt1 = 1;
             }
             double t1 = atan2(pt1, pt0);
@@ -3435,7 +3440,7 @@ __global__ void __launch_bounds__(128) k_rel2d_pairs(Rel2DArgs a)
                     break;
                 }
                 const double gr = hypot(og[2 * i], og[2 * i + 1]);
-                total += fabs((gr * s2) / den2) + fabs((gr * s1) / den1);
+                total += fabs(divide(gr * s2, den2)) + fabs(divide(gr * s1, den1));
             }
             if (!den_small) {
                 total *= (2 * a.approx_nf);
@@ -3527,7 +3532,7 @@ __global__ void k_cpdf1d_points(const double* tt, long long n, const double* xs,
             const double w2 = t[4] * t[4];
             double xms = x - t[5];
             xms *= xms;
-            fx += (t[6] * x + t[7]) / (w2 + xms);
+            fx += divide(t[6] * x + t[7], w2 + xms);
         }
         ys[q] = fx / fz;
     }

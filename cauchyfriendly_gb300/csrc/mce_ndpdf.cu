@@ -204,7 +204,8 @@ __device__ int nd_coalign(double* A, double* p, double* q, unsigned& hor, int m,
         double n1 = 0;
         for (int j = 0; j < LC; j++) n1 += fabs(A[i * LC + j]);
         p[i] *= n1;
-        for (int j = 0; j < LC; j++) A[i * LC + j] /= n1;
+        const DivBy by = div_by(n1);
+        for (int j = 0; j < LC; j++) A[i * LC + j] = divide(A[i * LC + j], by);
     }
     bool F[kNdMaxRows], hf[kNdMaxRows];
     for (int j = 0; j < m; j++) {
@@ -320,7 +321,8 @@ __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const doubl
             }
         }
         double mu_t[LC > 0 ? LC : 1];
-        for (int j = 0; j < LC; j++) mu_t[j] = A[tz * LD + j] / Ald[tz];
+        const DivBy by_t = div_by(Ald[tz]);
+        for (int j = 0; j < LC; j++) mu_t[j] = divide(A[tz * LD + j], by_t);
         double tb;
         double* bo = K.b + c * LC;
         if (x) {
@@ -338,7 +340,8 @@ __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const doubl
         for (int l = 0; l < m; l++) {
             if (l == tz) continue;
             if (nz[l]) {
-                for (int j = 0; j < LC; j++) Ac[l_ * LC + j] = A[l * LD + j] / Ald[l] - mu_t[j];
+                const DivBy by = div_by(Ald[l]);
+                for (int j = 0; j < LC; j++) Ac[l_ * LC + j] = divide(A[l * LD + j], by) - mu_t[j];
                 pc[l_] = pp[l] * fabs(Ald[l]);
             } else {
                 for (int j = 0; j < LC; j++) Ac[l_ * LC + j] = A[l * LD + j];
