@@ -545,9 +545,12 @@ public:
             return R;
         }
     } Rb;
-    DevBuf<cd> fam_mom, est_raw, scratch, g_vals, pr_gv;
+    DevBuf<cd> est_raw, scratch, g_vals, pr_gv;
     // post-FTR moments (print_basic_info): rows, chain totals, results
-    DevBuf<cd> pf_rows, pf_raw;
+    DevBuf<double> fam_mom, pf_rows;  // moment contributions, [component][row_pitch]
+    DevBuf<cd> pf_raw;
+    // rows of a contribution column: even, so that 16-byte copies stay aligned
+    static long long row_pitch(long long rows) { return (rows + 2) & ~1LL; }
     DevBuf<double> pf_tot, pf_gscale;
     DevBuf<long long> pf_zero;
     std::vector<cd> h_pf_raw;
@@ -1208,7 +1211,8 @@ public:
         const long long K = tot[0], Btot = tot[1], Kall = tot[2], Nvert = tot[3];
         const long long nR = nP + K;
         post_mu_terms += nP + Kall;
-        if ((s = fam_mom.ensure((size_t)(nP + Kall + 1) * (1 + D + D * D)))) return s;
+        const long long pitch = row_pitch(nP + Kall);
+        if ((s = fam_mom.ensure((size_t)pitch * 2 * (1 + D + D * D)))) return s;
         if ((s = Bkeys.ensure(Btot + 1))) return s;
         if ((s = vsv.ensure(Nvert + 1))) return s;
         if ((s = Rb.ensure(nR, MC))) return s;
@@ -1221,7 +1225,7 @@ public:
         if ((s = mu_ints.ensure((size_t)(nP + 1) * 4))) return s;
         pbeg(KID_MU);
         Kernels<D>::mu(PV, nP, dsteps.ptr, dpstart.ptr, droots.ptr, Told, Bkeys.ptr, R, nR, kall_scan.ptr, nP + Kall,
-                       mu_rows.ptr, mu_ints.ptr, fam_mom.ptr, MC, err, lc);
+                       mu_rows.ptr, mu_ints.ptr, fam_mom.ptr, pitch, MC, err, lc);
         pend();
         // the moment chains (and G_SCALE_FACTOR) on the side stream: the term
         // reduction below does not read them; the g-table evaluation does, so
@@ -1247,8 +1251,19 @@ public:
             LaunchCfg lcm = lc;
             lcm.stream = mstream;
             pbeg(KID_MOMENTS, mstream);
-            Kernels<D>::moments(fam_mom.ptr, dpstart.ptr, kall_scan.ptr, E, order, dsteps.ptr, mom_tot.ptr,
-                                est_raw.ptr, gscale.ptr, lcm);
+            // an estimator's rows: its parents and at most MC children of each
+            long long rows_lo = nP + Kall, rows_hi = nP + Kall;
+            if (E > 1) {
+                rows_hi = 0;
+                for (int e = 0; e < E; e++)
+                    if (hsteps[e].active) {
+                        const long long np = hpstart[e + 1] - hpstart[e];
+                        rows_lo = std::min(rows_lo, np);
+                        rows_hi = std::max(rows_hi, np * (MC + 1));
+                    }
+            }
+            Kernels<D>::moments(fam_mom.ptr, pitch, dpstart.ptr, kall_scan.ptr, E, order, dsteps.ptr, nP + Kall,
+                                rows_lo, rows_hi, mom_tot.ptr, est_raw.ptr, gscale.ptr, lcm);
             pend(mstream);
         }
         MCE_CUDA(cudaEventRecord(ev_join, mstream));
@@ -1618,16 +1633,17 @@ public:
         if (!any) return MCE_OK;
         constexpr int NM = 1 + D + D * D;
         int s;
-        if ((s = pf_rows.ensure((size_t)(nP + 1) * NM))) return s;
+        const long long pitch = row_pitch(nP);
+        if ((s = pf_rows.ensure((size_t)pitch * 2 * NM))) return s;
         if ((s = pf_zero.ensure(nP + 2))) return s;
         if ((s = pf_tot.ensure((size_t)E * 2 * NM))) return s;
         if ((s = pf_raw.ensure((size_t)E * NM))) return s;
         if ((s = pf_gscale.ensure(E))) return s;
         MCE_CUDA(cudaMemsetAsync(pf_zero.ptr, 0, sizeof(long long) * (nP + 2), lc.stream));
         Kernels<D>::post_ftr_terms(Pb[cur].view(), nP, droots.ptr, Tables{Tb[cur].keys.ptr, Tb[cur].vals.ptr}, MC,
-                                   pf_rows.ptr, lc);
-        Kernels<D>::moments(pf_rows.ptr, dpstart.ptr, pf_zero.ptr, E, nullptr, dsteps.ptr, pf_tot.ptr, pf_raw.ptr,
-                            pf_gscale.ptr, lc);
+                                   pf_rows.ptr, pitch, lc);
+        Kernels<D>::moments(pf_rows.ptr, pitch, dpstart.ptr, pf_zero.ptr, E, nullptr, dsteps.ptr, nP, 0,
+                            nP, pf_tot.ptr, pf_raw.ptr, pf_gscale.ptr, lc);
         h_pf_raw.resize((size_t)E * NM);
         h_pf_gscale.resize(E);
         MCE_CUDA(cudaMemcpyAsync(h_pf_raw.data(), pf_raw.ptr, sizeof(cd) * E * NM, cudaMemcpyDeviceToHost,

@@ -8,6 +8,7 @@
 // reduction group, member order, next parent order) is a rule on positions.
 #include "mce_kernels.cuh"
 #include "mce_c_api.h"
+#include "mce_chain.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -927,10 +928,9 @@ __global__ void __launch_bounds__(128) k_mu_terms(ParentList P, long long nP, co
                                                   const long long* pstart, const double* roots, Tables Told,
                                                   TermRecs R, long long nR, const long long* kall_scan,
                                                   long long nterms, const double* frow, const int* fint,
-                                                  cd* contrib, int MC, int* err)
+                                                  double* contrib, long long pitch, int MC, int* err)
 {
     extern __shared__ double smem_d[];
-    constexpr int NM = 1 + D + D * D;
     const int RS = MC * D + 2 * MC;
     const int FR = (MC + 1) * (D + 1) + 1;
     double* At = smem_d + (size_t)threadIdx.x * RS;
@@ -1031,13 +1031,18 @@ __global__ void __launch_bounds__(128) k_mu_terms(ParentList P, long long nP, co
         const double dv = rho[t];
         cd g = csub(cdiv(gp, mkcd(ygi + dv, zeta)), cdiv(gm, mkcd(ygi - dv, zeta)));
         g = cscale(g, kTwoPiInv);
-        cd* cs = contrib + xo * NM;
-        cs[0] = g;
+        // component by component: the rows of a warp's children are neighbours
+        double* cs = contrib + xo;
+        auto put = [&](int q, cd v) {
+            cs[(2 * q) * pitch] = v.re;
+            cs[(2 * q + 1) * pitch] = v.im;
+        };
+        put(0, g);
         for (int j = 0; j < D; j++) {
             const cd y = mkcd(-ty[j], bt[j]);
             const cd gy = cmul(g, y);
-            cs[1 + j] = gy;
-            for (int kk = 0; kk < D; kk++) cs[1 + D + j * D + kk] = cmul(gy, mkcd(-ty[kk], bt[kk]));
+            put(1 + j, gy);
+            for (int kk = 0; kk < D; kk++) put(1 + D + j * D + kk, cmul(gy, mkcd(-ty[kk], bt[kk])));
         }
         const long long pslot = i + P.kscan[pstart[e]];            // parent's record
         const long long cslot0 = pstart[e + 1] + P.kscan[i];       // first child's record
@@ -1094,40 +1099,19 @@ __global__ void __launch_bounds__(128) k_mu_terms(ParentList P, long long nP, co
     }
 }
 
-// Per-estimator moment sums, then finalize_cached_moments
-// (cauchy_estimator.hpp:340-357).  The reference accumulates fz, the mean and
-// the covariance in one sequential pass over the terms (parents in order, each
-// followed by its children); the same chain is summed here, so the moments
-// come out bit-identical to the serial reference.
+// Per-estimator moment sums in the reference's order (mce_chain.cuh), then
+// finalize_cached_moments (cauchy_estimator.hpp:340-357).
 //
-// The chains are independent per moment component: one warp per (estimator,
-// 32 components), each lane adding its component over the estimator's rows in
-// order.  A chain is a run of dependent additions, so the rows are streamed
-// into a shared-memory ring by cp.async ahead of the adder: with one active
-// estimator of 10^6 terms the chain runs at the FP64 add rate instead of
-// waiting on DRAM once every few rows.  Each lane copies and reads only its
-// own column, so its own cp.async.wait_group is the only synchronisation.
-constexpr int kMomStages = 3, kMomRows = 64;
-
-__device__ inline void cp_async8(double* smem_dst, const double* gmem_src)
-{
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem_src) : "memory");
-}
-__device__ inline void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ inline void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
+// k_moments_chain, a warp per (estimator, 32 components): the chains of fewer
+// than scan_rows rows.
 template <int D>
-__global__ void __launch_bounds__(32) k_moments_chain(const cd* contrib, const long long* pstart,
+__global__ void __launch_bounds__(32) k_moments_chain(const double* contrib, long long pitch, const long long* pstart,
                                                       const long long* kall_scan, int E, const int* order,
-                                                      const EstStep<D>* st, double* tot)
+                                                      const EstStep<D>* st, long long scan_rows, double* tot)
 {
-    constexpr int NM = 1 + D + D * D;
-    constexpr int ND = 2 * NM;              // doubles per term
-    constexpr int NS = (ND + 31) / 32;      // 32-component slices
-    __shared__ double ring[kMomStages][kMomRows][32];
-    const int lane = threadIdx.x;
+    constexpr int ND = 2 * (1 + D + D * D);  // doubles per term
+    constexpr int NS = (ND + 31) / 32;       // 32-component slices
+    __shared__ double2 ring[kMomStages][kMomRows / 2][32];
     const int eb = blockIdx.x / NS, slice = blockIdx.x - eb * NS;
     if (eb >= E) return;
     // blocks start in launch order: the longest chains go first
@@ -1135,77 +1119,58 @@ __global__ void __launch_bounds__(32) k_moments_chain(const cd* contrib, const l
     if (!st[e].active) return;
     const long long a = pstart[e] + kall_scan[pstart[e]];
     const long long n = pstart[e + 1] + kall_scan[pstart[e + 1]] - a;
-    const int comp = slice * 32 + lane;
+    if (n >= scan_rows) return;
+    const int comp = slice * 32 + threadIdx.x;
     const bool valid = comp < ND;
-    const double* col = reinterpret_cast<const double*>(contrib) + a * ND + comp;
-    const long long nchunks = (n + kMomRows - 1) / kMomRows;
-    // chunk k of this lane's column into ring slot k % kMomStages (one commit group per chunk)
-    auto issue = [&](long long k) {
-        if (valid && k < nchunks) {
-            const long long r0 = k * kMomRows;
-            const int cnt = n - r0 < kMomRows ? (int)(n - r0) : kMomRows;
-            double(*slot)[32] = ring[k % kMomStages];
-            const double* src = col + r0 * ND;
-            if (cnt == kMomRows) {
-#pragma unroll
-                for (int r = 0; r < kMomRows; r++) cp_async8(&slot[r][lane], src + r * ND);
-            } else
-                for (int r = 0; r < cnt; r++) cp_async8(&slot[r][lane], src + r * ND);
-        }
-        cp_async_commit();
-    };
-    for (int k = 0; k < kMomStages - 1; k++) issue(k);
-    double sum = 0.0;
-    for (long long k = 0; k < nchunks; k++) {
-        cp_async_wait<kMomStages - 2>();  // chunk k has landed
-        // refill the slot of chunk k - 1, whose values were added last iteration
-        issue(k + kMomStages - 1);
-        if (valid) {
-            const long long r0 = k * kMomRows;
-            const double(*slot)[32] = ring[k % kMomStages];
-            if (n - r0 >= kMomRows) {
-                // all loads first, then the dependent additions back to back
-                double v[kMomRows];
-#pragma unroll
-                for (int r = 0; r < kMomRows; r++) v[r] = slot[r][lane];
-#pragma unroll
-                for (int r = 0; r < kMomRows; r++) sum += v[r];
-            } else {
-                const int cnt = (int)(n - r0);
-                for (int r = 0; r < cnt; r++) sum += slot[r][lane];
-            }
-        }
-    }
-    cp_async_wait<0>();
+    const double sum = chain_short(valid ? contrib + comp * pitch : nullptr, a, n, ring);
     if (valid) tot[(long long)e * ND + comp] = sum;
 }
 
-// finalize_cached_moments (cauchy_estimator.hpp:340-357) from the chain totals.
+// k_moments_scan, a block per (estimator, component): the chains of scan_rows
+// rows or more.
+template <int D>
+__global__ void __launch_bounds__(kChainThreads) k_moments_scan(const double* contrib, long long pitch, const long long* pstart,
+                                                     const long long* kall_scan, int E, const int* order,
+                                                     const EstStep<D>* st, long long scan_rows, double* tot)
+{
+    constexpr int ND = 2 * (1 + D + D * D);
+    __shared__ ChainSmem sm;
+    const int eb = blockIdx.x / ND, comp = blockIdx.x - eb * ND;
+    if (eb >= E) return;
+    const int e = order ? order[eb] : eb;
+    if (!st[e].active) return;
+    const long long a = pstart[e] + kall_scan[pstart[e]];
+    const long long n = pstart[e + 1] + kall_scan[pstart[e + 1]] - a;
+    if (n < scan_rows) return;
+    const double sum = chain_scan(contrib + comp * pitch, a, n, sm);
+    if (threadIdx.x == 0) tot[(long long)e * ND + comp] = sum;
+}
+
+// finalize_cached_moments (cauchy_estimator.hpp:340-357) from the chain
+// totals, a thread per (estimator, moment): a covariance entry divides out its
+// two means again rather than waiting for their threads.
 template <int D>
 __global__ void k_moments_final(const double* tot, int E, const EstStep<D>* st, cd* est_raw, double* gscale)
 {
     constexpr int NM = 1 + D + D * D;
-    constexpr int ND = 2 * NM;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int e = (int)(x / NM), q = (int)(x - (long long)e * NM);
     if (e >= E || !st[e].active) return;
-    const double* t = tot + (long long)e * ND;
+    const double* t = tot + (long long)e * 2 * NM;
     const cd fz = mkcd(t[0], t[1]);
-    gscale[e] = kTwoPiInv / fz.re;
     const cd ifz = mkcd(0, fz.re);
-    cd* out = est_raw + (long long)e * NM;
-    out[0] = fz;
-    cd mfin[D];
-    for (int j = 0; j < D; j++) {
-        mfin[j] = cdiv(mkcd(t[2 * (1 + j)], t[2 * (1 + j) + 1]), ifz);
-        out[1 + j] = mfin[j];
+    cd* out = est_raw + (long long)e * NM + q;
+    auto mean = [&](int j) { return cdiv(mkcd(t[2 * (1 + j)], t[2 * (1 + j) + 1]), ifz); };
+    if (q == 0) {
+        gscale[e] = kTwoPiInv / fz.re;
+        *out = fz;
+    } else if (q <= D) {
+        *out = mean(q - 1);
+    } else {
+        // the covariance is accumulated as cov -= (g y_j) y_k, i.e. minus the chain
+        const int j = (q - 1 - D) / D, k = (q - 1 - D) - j * D;
+        *out = csub(cdiv(mkcd(-t[2 * q], -t[2 * q + 1]), fz), cmul(mean(j), mean(k)));
     }
-    // the covariance is accumulated as cov -= (g y_j) y_k, i.e. minus the chain
-    for (int j = 0; j < D; j++)
-        for (int k = 0; k < D; k++) {
-            const int q = 2 * (1 + D + j * D + k);
-            const cd cv = mkcd(-t[q], -t[q + 1]);
-            out[1 + D + j * D + k] = csub(cdiv(cv, fz), cmul(mfin[j], mfin[k]));
-        }
 }
 
 // ---------------------------------------------------------------------------
@@ -2547,7 +2512,7 @@ void Kernels<D>::build_B(ParentList P, long long nP, const EstStep<D>* st, int w
 template <int D>
 void Kernels<D>::mu(ParentList P, long long nP, const EstStep<D>* st, const long long* pstart, const double* roots,
                     Tables Told, int* Bkeys, TermRecs R, long long nR, const long long* kall_scan, long long nterms,
-                    double* frow, int* fint, cd* contrib, int MC, int* err, const LaunchCfg& c)
+                    double* frow, int* fint, double* contrib, long long pitch, int MC, int* err, const LaunchCfg& c)
 {
     if (nP == 0) return;
     ++g_launches;
@@ -2568,18 +2533,46 @@ void Kernels<D>::mu(ParentList P, long long nP, const EstStep<D>* st, const long
     cudaFuncSetAttribute(k_mu_terms<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     ++g_launches;
     k_mu_terms<D><<<grid_for(nterms, threads, c.num_sms, 16), threads, sm, c.stream>>>(
-        P, nP, st, pstart, roots, Told, R, nR, kall_scan, nterms, frow, fint, contrib, MC, err);
+        P, nP, st, pstart, roots, Told, R, nR, kall_scan, nterms, frow, fint, contrib, pitch, MC, err);
 }
 
+// Chains of scan_rows rows or more take the scan.  It spends about five FP64
+// instructions where chain_short spends one, to run several rows at once, so
+// it pays while its blocks (one per estimator and component) leave the SMs'
+// FP64 pipes idle: up to kChainBlocksPerSm of them per SM, from one tile's
+// quarter on (256 rows: 2.5 us against 8).  Measured on recorded contributions
+// of one estimator: 36,056 rows x 42 components 0.39 ms against 1.59, 30,982 x
+// 62 0.30 against 1.37 (5 ns a row, 10 on the imaginary part of fz, whose sum
+// returns to rounding noise after every family).  With more estimators the
+// short chains fill the pipes (4,096 estimators, 54 M rows a pass: 8.8 ms;
+// with the scan for the chains of 4,096 rows or more 25 ms), and only a chain
+// that holds a kChainScanShare-th of all rows is worth it.
+constexpr long long kChainBlocksPerSm = 8;
+constexpr long long kChainScanRowsFew = 256, kChainScanRowsMany = 4096, kChainScanShare = 64;
+
 template <int D>
-void Kernels<D>::moments(const cd* contrib, const long long* pstart, const long long* kall_scan, int E,
-                         const int* order, const EstStep<D>* st, double* tot, cd* est_raw, double* gscale,
-                         const LaunchCfg& c)
+void Kernels<D>::moments(const double* contrib, long long pitch, const long long* pstart, const long long* kall_scan,
+                         int E, const int* order, const EstStep<D>* st, long long rows, long long rows_lo,
+                         long long rows_hi, double* tot, cd* est_raw, double* gscale, const LaunchCfg& c)
 {
-    constexpr int NS = (2 * (1 + D + D * D) + 31) / 32;
-    g_launches += 2;
-    k_moments_chain<D><<<(unsigned)E * NS, 32, 0, c.stream>>>(contrib, pstart, kall_scan, E, order, st, tot);
-    k_moments_final<D><<<(E + 127) / 128, 128, 0, c.stream>>>(tot, E, st, est_raw, gscale);
+    constexpr int ND = 2 * (1 + D + D * D);
+    constexpr int NS = (ND + 31) / 32;
+    const long long scan_rows = (long long)E * ND <= kChainBlocksPerSm * c.num_sms
+                                    ? kChainScanRowsFew
+                                    : std::max(kChainScanRowsMany, rows / kChainScanShare);
+    if (rows_lo < scan_rows) {
+        ++g_launches;
+        k_moments_chain<D><<<(unsigned)E * NS, 32, 0, c.stream>>>(contrib, pitch, pstart, kall_scan, E, order, st,
+                                                                  scan_rows, tot);
+    }
+    if (rows_hi >= scan_rows) {
+        ++g_launches;
+        k_moments_scan<D><<<(unsigned)E * ND, kChainThreads, 0, c.stream>>>(contrib, pitch, pstart, kall_scan, E,
+                                                                            order, st, scan_rows, tot);
+    }
+    ++g_launches;
+    k_moments_final<D><<<(unsigned)(((long long)E * (ND / 2) + 127) / 128), 128, 0, c.stream>>>(tot, E, st, est_raw,
+                                                                                               gscale);
 }
 
 template <int D>
@@ -3458,9 +3451,9 @@ __global__ void __launch_bounds__(128) k_rel2d_pairs(Rel2DArgs a)
 // yei = -sum p_l s_l A_l + i b -- into a moment row laid out as k_mu_terms
 // writes them (g, g y_j, g y_j y_k), for the same chain and finalisation.
 template <int D>
-__global__ void k_post_ftr_terms(ParentList P, long long nP, const double* roots, Tables T, int MC, cd* contrib)
+__global__ void k_post_ftr_terms(ParentList P, long long nP, const double* roots, Tables T, int MC, double* contrib,
+                                 long long pitch)
 {
-    constexpr int NM = 1 + D + D * D;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nP;
          i += (long long)gridDim.x * blockDim.x) {
         const int e = P.est[i];
@@ -3480,23 +3473,28 @@ __global__ void k_post_ftr_terms(ParentList P, long long nP, const double* roots
             if (!sp) enc |= 1 << l;
         }
         const cd g = lookup_num(T.keys + P.tab_off[i], T.vals + P.tab_off[i], P.tab_cnt[i], enc, m);
-        cd* cs = contrib + i * NM;
-        cs[0] = g;
+        double* cs = contrib + i;
+        auto put = [&](int q, cd v) {
+            cs[(2 * q) * pitch] = v.re;
+            cs[(2 * q + 1) * pitch] = v.im;
+        };
+        put(0, g);
         for (int j = 0; j < D; j++) {
             const cd gy = cmul(g, mkcd(-ty[j], P.b[i * D + j]));
-            cs[1 + j] = gy;
-            for (int k = 0; k < D; k++) cs[1 + D + j * D + k] = cmul(gy, mkcd(-ty[k], P.b[i * D + k]));
+            put(1 + j, gy);
+            for (int k = 0; k < D; k++) put(1 + D + j * D + k, cmul(gy, mkcd(-ty[k], P.b[i * D + k])));
         }
     }
 }
 
 template <int D>
-void Kernels<D>::post_ftr_terms(ParentList P, long long nP, const double* roots, Tables T, int MC, cd* contrib,
-                                const LaunchCfg& c)
+void Kernels<D>::post_ftr_terms(ParentList P, long long nP, const double* roots, Tables T, int MC, double* contrib,
+                                long long pitch, const LaunchCfg& c)
 {
     if (nP == 0) return;
     ++g_launches;
-    k_post_ftr_terms<D><<<grid_for(nP, 128, c.num_sms, 16), 128, 0, c.stream>>>(P, nP, roots, T, MC, contrib);
+    k_post_ftr_terms<D><<<grid_for(nP, 128, c.num_sms, 16), 128, 0, c.stream>>>(P, nP, roots, T, MC, contrib,
+                                                                                     pitch);
 }
 
 template <int D>

@@ -165,14 +165,17 @@ struct Kernels {
     // Measurement update, g/yei evaluation, moment partials, MU coalignment.
     static void mu(ParentList P, long long nP, const EstStep<D>* st, const long long* pstart,
                    const double* roots, Tables Told, int* Bkeys, TermRecs R, long long nR,
-                   const long long* kall_scan, long long nterms, double* frow, int* fint, cd* contrib, int MC,
+                   const long long* kall_scan, long long nterms, double* frow, int* fint, double* contrib,
+                   long long pitch, int MC,
                    int* err, const LaunchCfg& c);
     // Per-estimator moment sums in the reference's order and finalisation
-    // (cauchy_estimator.hpp:307-357); the chains start in the estimator order
-    // given by order (null: 0..E-1), longest first when the caller sorts.
-    static void moments(const cd* contrib, const long long* pstart, const long long* kall_scan, int E,
-                        const int* order, const EstStep<D>* st, double* tot, cd* est_raw, double* gscale,
-                        const LaunchCfg& c);
+    // (cauchy_estimator.hpp:307-357) over contrib[component * pitch + row];
+    // the chains start in the estimator order given by order (null: 0..E-1),
+    // longest first when the caller sorts.  rows: all of them; rows_lo,
+    // rows_hi: bounds on an active estimator's.
+    static void moments(const double* contrib, long long pitch, const long long* pstart, const long long* kall_scan,
+                        int E, const int* order, const EstStep<D>* st, long long rows, long long rows_lo,
+                        long long rows_hi, double* tot, cd* est_raw, double* gscale, const LaunchCfg& c);
     // Fast term reduction (term_reduction.hpp:159-276) over the post-MU records:
     // grid cells of b, counting-sorted buckets, near predecessors.
     static void ftr_cells(TermRecs R, long long nR, long long hmask, int* slot_of, int* bcount, const LaunchCfg& c);
@@ -243,8 +246,8 @@ struct Kernels {
                             const double* gscale, const long long* toff, Tables Tnew, const GFlat& f, int MC,
                             const LaunchCfg& c);
     // Moment rows of the current (reduced) terms, compute_moments(false).
-    static void post_ftr_terms(ParentList P, long long nP, const double* roots, Tables T, int MC, cd* contrib,
-                               const LaunchCfg& c);
+    static void post_ftr_terms(ParentList P, long long nP, const double* roots, Tables T, int MC,
+                               double* contrib, long long pitch, const LaunchCfg& c);
     // One relative 2-D term per (primary term, secondary term) pair: its
     // cache row, kept flag and moment contributions.
     static void rel2d_pairs(const Rel2DArgs& a, const LaunchCfg& c);
