@@ -1710,7 +1710,7 @@ public:
     std::vector<int> cpdf2_step, cpdf2_i1, cpdf2_i2;
     std::vector<long long> cpdf2_n;
     std::vector<std::unique_ptr<DevBuf<double>>> cpdf2_tt;
-    DevBuf<double> cpdf2_x, cpdf2_y, cpdf2_z;
+    DevBuf<double> cpdf2_x, cpdf2_y, cpdf2_z, cpdf_part;
 
     int cpdf_2d_grid(int e, int i1, int i2, const double* bar_nu, double lx, double hx, double rx, double ly,
                      double hy, double ry, int reset_cache, int max_points, double* xs, double* ys,
@@ -1780,8 +1780,10 @@ public:
         MCE_CUDA(cudaMemcpyAsync(cpdf2_x.ptr, xs, sizeof(double) * npts, cudaMemcpyHostToDevice, lc.stream));
         MCE_CUDA(cudaMemcpyAsync(cpdf2_y.ptr, ys, sizeof(double) * npts, cudaMemcpyHostToDevice, lc.stream));
         MCE_CUDA(cudaMemsetAsync(counters.ptr + 7, 0, sizeof(int), lc.stream));
-        cpdf2d_points(cpdf2_tt[e]->ptr, n, MC, cpdf2_x.ptr, cpdf2_y.ptr, npts, est[e].fz[0], cpdf2_z.ptr,
-                      counters.ptr + 7, lc);
+        const PdfChunks pc = pdf_chunks(n, npts, 2, lc);
+        if ((s = cpdf_part.ensure((size_t)npts * pc.nch))) return s;
+        cpdf2d_points(cpdf2_tt[e]->ptr, n, MC, cpdf2_x.ptr, cpdf2_y.ptr, npts, est[e].fz[0], pc, cpdf_part.ptr,
+                      cpdf2_z.ptr, counters.ptr + 7, lc);
         int bad = 0;
         MCE_CUDA(cudaMemcpyAsync(zs, cpdf2_z.ptr, sizeof(double) * npts, cudaMemcpyDeviceToHost, lc.stream));
         MCE_CUDA(cudaMemcpyAsync(&bad, counters.ptr + 7, sizeof(int), cudaMemcpyDeviceToHost, lc.stream));
@@ -1993,7 +1995,9 @@ public:
         if ((s = cpdf_x.ensure(npts))) return s;
         if ((s = cpdf_y.ensure(npts))) return s;
         MCE_CUDA(cudaMemcpyAsync(cpdf_x.ptr, xs, sizeof(double) * npts, cudaMemcpyHostToDevice, lc.stream));
-        cpdf1d_points(cpdf_tt[e]->ptr, n, cpdf_x.ptr, npts, exact, est[e].fz[0], cpdf_y.ptr, lc);
+        const PdfChunks pc = pdf_chunks(n, npts, 1, lc);
+        if ((s = cpdf_part.ensure((size_t)npts * pc.nch))) return s;
+        cpdf1d_points(cpdf_tt[e]->ptr, n, cpdf_x.ptr, npts, exact, est[e].fz[0], pc, cpdf_part.ptr, cpdf_y.ptr, lc);
         MCE_CUDA(cudaMemcpyAsync(ys, cpdf_y.ptr, sizeof(double) * npts, cudaMemcpyDeviceToHost, lc.stream));
         MCE_CUDA(cudaStreamSynchronize(lc.stream));
         return npts;
@@ -2450,21 +2454,13 @@ int rel2d_grid(mce_rel2d* r, double xlow, double xhigh, double dx, double ylow, 
             y[i * ny + j] = j == ny - 1 ? yhigh : ylow + dy * j;
         }
     }
-    // enough (point, chunk) threads for two full waves, chunks of at least 32
-    // kept terms; one chunk keeps the reference's summation order exactly
     const long long nk = r->nkept;
-    long long nch = ((long long)r->lc.num_sms * 2048 * 2 + npts - 1) / npts;
-    const long long maxch = (nk + 31) / 32;
-    if (nch > maxch) nch = maxch;
-    if (nch < 1) nch = 1;
-    if (nch > 65535) nch = 65535;
-    long long chunk = nk > 0 ? (nk + nch - 1) / nch : 1;
-    nch = nk > 0 ? (nk + chunk - 1) / chunk : 1;
+    const PdfChunks pc = pdf_chunks(nk, npts, 2, r->lc);
     int s;
     if ((s = r->xs.ensure(npts))) return s;
     if ((s = r->ys.ensure(npts))) return s;
     if ((s = r->zs.ensure(npts))) return s;
-    if ((s = r->part.ensure((size_t)nch * npts))) return s;
+    if ((s = r->part.ensure((size_t)pc.nch * npts))) return s;
     if ((s = r->bad.ensure(1))) return s;
     cudaStream_t st = r->stream;
     MCE_CUDA(cudaMemcpyAsync(r->xs.ptr, x, sizeof(double) * npts, cudaMemcpyHostToDevice, st));
@@ -2472,9 +2468,8 @@ int rel2d_grid(mce_rel2d* r, double xlow, double xhigh, double dx, double ylow, 
     MCE_CUDA(cudaMemsetAsync(r->bad.ptr, 0, sizeof(int), st));
     MCE_CUDA(cudaEventRecord(r->ev[4], st));
     r->launches += 2;
-    rel2d_points(r->tt.ptr, r->kidx.ptr, nk, r->CC, r->full, chunk, (int)nch, r->xs.ptr, r->ys.ptr, npts,
-                 r->part.ptr, r->bad.ptr, r->lc);
-    rel2d_finish(r->part.ptr, (int)nch, npts, r->full, nf_prim, nf_sec, r->zs.ptr, r->lc);
+    rel2d_points(r->tt.ptr, r->kidx.ptr, nk, r->CC, r->full, r->xs.ptr, r->ys.ptr, npts, nf_prim * nf_sec, pc,
+                 r->part.ptr, r->zs.ptr, r->bad.ptr, r->lc);
     MCE_CUDA(cudaEventRecord(r->ev[5], st));
     MCE_CUDA(cudaGetLastError());
     int bad = 0;

@@ -3032,8 +3032,25 @@ void Kernels<D>::det_tp(ParentList P, long long a, long long n, const double* Ph
 // the real parts of gamma1, gamma2 (:1551-1600).  This is the reference's
 // per-term cache (Cached2DCPDFTerm); its exact first evaluation uses the same
 // sines, cosines and gammas, so every grid point is summed from the cache.
-// Record per term (cpdf2d_stride doubles): m, b1, b2, sin[MC+1], cos[MC+1],
-// g1r[MC], g2r[MC], g[MC] (re, im).
+// The record: marg2d_term.
+
+// One cell of a record: its first wall's direction (s, c), the real parts of
+// gamma1 and gamma2, the g value.
+__device__ inline void marg2d_put_cell(double* o, int c, double s, double co, double g1r, double g2r, cd g)
+{
+    double* w = o + 3 + 6 * c;
+    w[0] = s;
+    w[1] = co;
+    w[2] = g1r;
+    w[3] = g2r;
+    w[4] = g.re;
+    w[5] = g.im;
+}
+__device__ inline void marg2d_put_last_wall(double* o, int cells, double s, double co)
+{
+    o[3 + 6 * cells] = s;
+    o[4 + 6 * cells] = co;
+}
 
 template <int D>
 __global__ void k_cpdf2d_terms(ParentList P, long long a, long long n, int i1, int i2, const double* bar_nu, Tables T,
@@ -3128,17 +3145,17 @@ __global__ void k_cpdf2d_terms(ParentList P, long long a, long long n, int i1, i
             th[y + 1] = v;
         }
         double* o = tt + q * RT;
-        double* os = o + 3;
-        double* oc = os + (MC + 1);
-        double* o1 = oc + (MC + 1);
-        double* o2 = o1 + MC;
-        double* og = o2 + MC;
         o[0] = mn;
         o[1] = P.b[i * D + i1];
         o[2] = P.b[i * D + i2];
         const int* keys = T.keys + P.tab_off[i];
         const cd* vals = T.vals + P.tab_off[i];
         const int cnt = P.tab_cnt[i];
+        double s1 = 0, c1 = 0;
+        if (mn > 0) {
+            s1 = sin(th[0]);
+            c1 = cos(th[0]);
+        }
         for (int c = 0; c < mn; c++) {
             const double tm = (th[c + 1] + th[c]) / 2.0;
             const double ct = cos(tm), st = sin(tm);
@@ -3167,15 +3184,12 @@ __global__ void k_cpdf2d_terms(ParentList P, long long a, long long n, int i1, i
                 g1r -= (A2[2 * j] * p2[j]) * sv;
                 g2r -= (A2[2 * j + 1] * p2[j]) * sv;
             }
-            os[c] = sin(th[c]);
-            oc[c] = cos(th[c]);
-            o1[c] = g1r;
-            o2[c] = g2r;
-            og[2 * c] = g.re;
-            og[2 * c + 1] = g.im;
+            const double s2 = sin(th[c + 1]), c2 = cos(th[c + 1]);
+            marg2d_put_cell(o, c, s1, c1, g1r, g2r, g);
+            s1 = s2;
+            c1 = c2;
         }
-        os[mn] = mn > 0 ? sin(th[mn]) : 0.0;
-        oc[mn] = mn > 0 ? cos(th[mn]) : 0.0;
+        marg2d_put_last_wall(o, mn, s1, c1);
     }
 }
 
@@ -3381,14 +3395,14 @@ __global__ void __launch_bounds__(128) k_rel2d_pairs(Rel2DArgs a)
         if (a.full && mn > 0) th[2 * mn] = th[0] + 2 * kPi;
         const int cells = mn * (1 + a.full);
         double* o = a.tt + x * RT;
-        double* os = o + 3;
-        double* oc = os + (a.CC + 1);
-        double* o1 = oc + (a.CC + 1);
-        double* o2 = o1 + a.CC;
-        double* og = o2 + a.CC;
         o[0] = mn;
         o[1] = b2[0];
         o[2] = b2[1];
+        // approx_out_rel_marg2d_term_for_cpdf (:445-470), cell by cell
+        double total = 0;
+        bool den_small = false;
+        double s1 = 0, c1 = 0;
+        if (cells > 0) sincos(th[0], &s1, &c1);
         const unsigned allm = mn >= 32 ? 0xffffffffu : ((1u << mn) - 1u);
         for (int c = 0; c < cells; c++) {
             const int h = c < mn ? c : c - mn;
@@ -3412,33 +3426,27 @@ __global__ void __launch_bounds__(128) k_rel2d_pairs(Rel2DArgs a)
                 g1r -= (Ac[2 * j] * pc[j]) * sv;
                 g2r -= (Ac[2 * j + 1] * pc[j]) * sv;
             }
-            sincos(th[c], os + c, oc + c);
-            o1[c] = g1r;
-            o2[c] = g2r;
-            og[2 * c] = g.re;
-            og[2 * c + 1] = g.im;
-        }
-        if (cells > 0) sincos(th[cells], os + cells, oc + cells);
-        else os[0] = oc[0] = 0.0;
-        int keep = 1;
-        if (a.approx) {
-            double total = 0;
-            bool den_small = false;
-            for (int i = 0; i < mn; i++) {
-                const double a1 = o1[i], a2 = o2[i], c1 = oc[i], s1 = os[i], c2 = oc[i + 1], s2 = os[i + 1];
-                const double den1 = a1 * (a1 * c1 + a2 * s1);
-                const double den2 = a1 * (a1 * c2 + a2 * s2);
+            double s2, c2;
+            sincos(th[c + 1], &s2, &c2);
+            marg2d_put_cell(o, c, s1, c1, g1r, g2r, g);
+            if (a.approx && c < mn && !den_small) {
+                const double den1 = g1r * (g1r * c1 + g2r * s1);
+                const double den2 = g1r * (g1r * c2 + g2r * s2);
                 if (fabs(den1) < 1e-14 || fabs(den2) < 1e-14) {
                     den_small = true;
-                    break;
+                } else {
+                    const double gr = hypot(g.re, g.im);
+                    total += fabs(divide(gr * s2, den2)) + fabs(divide(gr * s1, den1));
                 }
-                const double gr = hypot(og[2 * i], og[2 * i + 1]);
-                total += fabs(divide(gr * s2, den2)) + fabs(divide(gr * s1, den1));
             }
-            if (!den_small) {
-                total *= (2 * a.approx_nf);
-                if (fabs(total) < a.eps) keep = 0;
-            }
+            s1 = s2;
+            c1 = c2;
+        }
+        marg2d_put_last_wall(o, cells, s1, c1);
+        int keep = 1;
+        if (a.approx && !den_small) {
+            total *= (2 * a.approx_nf);
+            if (fabs(total) < a.eps) keep = 0;
         }
         a.keep[x] = keep;
     }
@@ -3506,40 +3514,63 @@ void Kernels<D>::rel2d_pairs(const Rel2DArgs& a, const LaunchCfg& c)
 }
 
 #if MCE_COMMON_UNIT
-// One thread per point, the terms summed in order.  Points below `exact`
-// take the complex formula (fx * 1/(2 pi) / fz), the others the cached one
-// (fx / fz).
-__global__ void k_cpdf1d_points(const double* tt, long long n, const double* xs, int npts, int exact, double fz,
-                                double* ys)
+// The pdf grids: a thread per (point, chunk of terms), the chunk summed in
+// order into part[chunk * npts + point]; then a warp per point adds its chunks.
+// A thread per point alone left the chip idle (801 points: 13 blocks of 64
+// threads, each walking 3,324 terms at the latency of a dependent addition):
+// that curve went from 2,726 to 89 us a call, 101 x 83 points of a surface of
+// 465 terms from 4,531 to 1,035 us.
+//
+// 1-D.  Points below `exact` take the complex formula (fx * 1/(2 pi) / fz),
+// the others the cached one (fx / fz).
+__global__ void k_cpdf1d_points(const double* tt, long long n, const double* xs, int npts, int exact, long long chunk,
+                                int nch, double* part)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npts) return;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)npts * nch) return;
+    const int ch = (int)(i / npts), q = (int)(i - (long long)ch * npts);
+    const long long j0 = ch * chunk, j1 = j0 + chunk < n ? j0 + chunk : n;
     const double x = xs[q];
     double fx = 0;
     if (q < exact) {
-        for (long long j = 0; j < n; j++) {
+        for (long long j = j0; j < j1; j++) {
             const double* t = tt + j * 8;
             const double b_c = t[5] - x;
             const cd g = csub(cdiv(mkcd(t[0], t[1]), mkcd(t[4], b_c)), cdiv(mkcd(t[2], t[3]), mkcd(-t[4], b_c)));
             fx += g.re;
         }
-        ys[q] = fx * kTwoPiInv / fz;
     } else {
-        for (long long j = 0; j < n; j++) {
+        for (long long j = j0; j < j1; j++) {
             const double* t = tt + j * 8;
             const double w2 = t[4] * t[4];
             double xms = x - t[5];
             xms *= xms;
             fx += divide(t[6] * x + t[7], w2 + xms);
         }
-        ys[q] = fx / fz;
     }
+    part[i] = fx;
+}
+
+// x / y for a real x: cdiv(mkcd(x, 0), y) without the operations on the zero
+// (x + 0, 0 - x and their like change no bit of a nonzero value).
+__device__ inline cd rdiv(double x, cd y)
+{
+    const double c = y.re, d = y.im;
+    const bool big_c = !(dabs_bits(c) < dabs_bits(d));
+    const double p = big_c ? c : d, q = big_c ? d : c;
+    const double r = divide(q, p);
+    const DivBy by = div_by(q * r + p);
+    const double u = divide(x, by), v = divide(x * r, by);
+    return big_c ? cd{u, -v} : cd{v, -u};
 }
 
 // One cell's integral (marg2d_eval_term_for_cpdf / marg2d_cached_eval_term_for_cpdf,
 // cpdf_ndim.hpp:1602-1640, 1710-1740): the fast form, or, with gamma1 ~ 0,
 // the form that also handles gamma2 ~ 0; both ~ 0 is the reference's exit,
-// reported here through *bad.
+// reported here through *bad.  The operations are the reference's: its
+// difference of the two walls cancels, and in the tails the values it gives
+// are off by more than the 1e-9 they are compared at (the algebraically equal
+// g sin(width) / (D1 D2) is closer to the truth there and too far from it).
 __device__ inline double marg2d_cell(double s1, double c1, double s2, double c2, double g1r, double g1i, double g2r,
                                      double g2i, bool check, cd g, int* bad)
 {
@@ -3556,8 +3587,8 @@ __device__ inline double marg2d_cell(double s1, double c1, double s2, double c2,
     if (fast) {
         gamma2 = cmul(gamma2, gamma1);
         gamma1 = cmul(gamma1, gamma1);
-        const cd lo = cdiv(mkcd(s1, 0), cadd(cscale(gamma1, c1), cscale(gamma2, s1)));
-        const cd hi = cdiv(mkcd(s2, 0), cadd(cscale(gamma1, c2), cscale(gamma2, s2)));
+        const cd lo = rdiv(s1, cadd(cscale(gamma1, c1), cscale(gamma2, s1)));
+        const cd hi = rdiv(s2, cadd(cscale(gamma1, c2), cscale(gamma2, s2)));
         cell = cmul(csub(hi, lo), g);
     } else {
         const cd lo = cdiv(csub(cscale(gamma1, s1), cscale(gamma2, c1)), cadd(cscale(gamma1, c1), cscale(gamma2, s1)));
@@ -3570,105 +3601,105 @@ __device__ inline double marg2d_cell(double s1, double c1, double s2, double c2,
     return cell.re;
 }
 
-// A thread per grid point; terms and their cells summed in order, then
-// 2 fx / (2 pi)^2 / fz (cpdf_ndim.hpp:1447).
-__global__ void k_cpdf2d_points(const double* tt, long long n, int MC, const double* xs, const double* ys, int npts,
-                                double fz, double* zs, int* bad)
+// A 2-D record's cells at one point.  Record: m, b1, b2, then per cell
+// (s, c, g1r, g2r, g re, g im) and the last wall's (s, c).
+__device__ inline double marg2d_term(const double* o, int cells, double x1, double x2, int* bad)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npts) return;
-    const int RT = cpdf2d_stride(MC);
-    const double x1 = xs[q], x2 = ys[q];
-    double fx = 0;
-    int b = 0;
-    for (long long j = 0; j < n; j++) {
-        const double* o = tt + j * RT;
-        const int mn = (int)o[0];
-        const double* os = o + 3;
-        const double* oc = os + (MC + 1);
-        const double* o1 = oc + (MC + 1);
-        const double* o2 = o1 + MC;
-        const double* og = o2 + MC;
-        const double g1i = o[1] - x1, g2i = o[2] - x2;
-        const bool check = fabs(g1i) < 1e-8;
-        double t = 0;
-        for (int c = 0; c < mn; c++)
-            t += marg2d_cell(os[c], oc[c], os[c + 1], oc[c + 1], o1[c], g1i, o2[c], g2i, check,
-                             mkcd(og[2 * c], og[2 * c + 1]), &b);
-        fx += t;
-    }
-    zs[q] = 2 * fx * kTwoPiInv * kTwoPiInv / fz;
-    if (b) atomicOr(bad, 1);
+    const double g1i = o[1] - x1, g2i = o[2] - x2;
+    const bool check = fabs(g1i) < 1e-8;
+    const double* w = o + 3;
+    double t = 0;
+    for (int c = 0; c < cells; c++, w += 6)
+        t += marg2d_cell(w[0], w[1], w[6], w[7], w[2], g1i, w[3], g2i, check, mkcd(w[4], w[5]), bad);
+    return t;
 }
 
-void cpdf2d_points(const double* tt, long long n, int MC, const double* xs, const double* ys, int npts, double fz,
-                   double* zs, int* bad, const LaunchCfg& c)
+// 2-D over the records tt (kidx null) or the kept records kidx[0..n), RT
+// doubles each; `mult` cells per counted row.
+__global__ void __launch_bounds__(128) k_cpdf2d_points(const double* tt, const long long* kidx, long long n, int RT,
+                                                       int mult, const double* xs, const double* ys, int npts,
+                                                       long long chunk, int nch, double* part, int* bad)
 {
-    if (npts <= 0) return;
-    ++g_launches;
-    k_cpdf2d_points<<<(npts + 63) / 64, 64, 0, c.stream>>>(tt, n, MC, xs, ys, npts, fz, zs, bad);
-}
-
-void cpdf1d_points(const double* tt, long long n, const double* xs, int npts, int exact, double fz, double* ys,
-                   const LaunchCfg& c)
-{
-    if (npts <= 0) return;
-    ++g_launches;
-    k_cpdf1d_points<<<(npts + 63) / 64, 64, 0, c.stream>>>(tt, n, xs, npts, exact, fz, ys);
-}
-
-// Relative 2-D pdf (eval_marg2d_relative_and_transformed_cpdf,
-// cauchy_prediction.hpp:973-1073): a thread per (grid point, chunk of pairs),
-// the chunk's kept terms and their cells summed in order; the integral of a
-// cell is the marginal 2-D one.
-__global__ void k_rel2d_points(const double* tt, const long long* kidx, long long nk, int CC, int full,
-                               long long chunk, const double* xs, const double* ys, int npts, double* part, int* bad)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= npts) return;
-    const long long j0 = (long long)blockIdx.y * chunk;
-    const long long j1 = j0 + chunk < nk ? j0 + chunk : nk;
-    const int RT = rel2d_stride(CC);
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)npts * nch) return;
+    const int ch = (int)(i / npts), q = (int)(i - (long long)ch * npts);
+    const long long j0 = ch * chunk, j1 = j0 + chunk < n ? j0 + chunk : n;
     const double x1 = xs[q], x2 = ys[q];
     double fx = 0;
     int b = 0;
     for (long long j = j0; j < j1; j++) {
-        const double* o = tt + kidx[j] * RT;
-        const int cells = (int)o[0] * (1 + full);
-        const double* os = o + 3;
-        const double* oc = os + (CC + 1);
-        const double* o1 = oc + (CC + 1);
-        const double* o2 = o1 + CC;
-        const double* og = o2 + CC;
-        const double g1i = o[1] - x1, g2i = o[2] - x2;
-        const bool check = fabs(g1i) < 1e-8;
-        double t = 0;
-        for (int c = 0; c < cells; c++)
-            t += marg2d_cell(os[c], oc[c], os[c + 1], oc[c + 1], o1[c], g1i, o2[c], g2i, check,
-                             mkcd(og[2 * c], og[2 * c + 1]), &b);
-        fx += t;
+        const double* o = tt + (kidx ? kidx[j] : j) * RT;
+        const int cells = (int)o[0] * mult;
+        fx += marg2d_term(o, cells, x1, x2, &b);
     }
-    part[(long long)blockIdx.y * npts + q] = fx;
+    part[i] = fx;
     if (b) atomicOr(bad, 1);
 }
 
-__global__ void k_rel2d_finish(const double* part, int nch, int npts, int full, double nf_prim, double nf_sec,
-                               double* zs)
+// out[q] = (the sum of point q's chunks) * scale / fz, `first` points with
+// scale0: a warp per point, the lanes' partial sums added in a fixed tree.
+__global__ void k_pdf_finish(const double* part, int nch, int npts, int first, double scale0, double scale1,
+                             double scale2, double fz, double* out)
 {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const int q = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (q >= npts) return;
     double fx = 0;
-    for (int ch = 0; ch < nch; ch++) fx += part[(long long)ch * npts + q];
-    zs[q] = ((double)(2 - full)) * fx * kTwoPiInv * kTwoPiInv / (nf_prim * nf_sec);
+    for (int ch = lane; ch < nch; ch += 32) fx += part[(long long)ch * npts + q];
+    for (int o = 16; o > 0; o >>= 1) fx += __shfl_down_sync(kFull, fx, o);
+    if (lane == 0) out[q] = (q < first ? fx * scale0 : scale1 * fx * scale2 * scale2) / fz;
 }
 
-void rel2d_points(const double* tt, const long long* kidx, long long nk, int CC, int full, long long chunk,
-                  int nch, const double* xs, const double* ys, int npts, double* part, int* bad, const LaunchCfg& c)
+// Chunks per point: about `waves` waves of 2,048 threads an SM, at least 8
+// terms a chunk.
+PdfChunks pdf_chunks(long long n, int npts, int waves, const LaunchCfg& c)
+{
+    PdfChunks k;
+    long long nch = ((long long)c.num_sms * 2048 * waves + npts - 1) / npts;
+    const long long maxch = (n + 7) / 8;
+    if (nch > maxch) nch = maxch;
+    if (nch < 1) nch = 1;
+    k.chunk = n > 0 ? (n + nch - 1) / nch : 1;
+    k.nch = n > 0 ? (int)((n + k.chunk - 1) / k.chunk) : 1;
+    return k;
+}
+
+static inline unsigned pdf_blocks(long long threads) { return (unsigned)((threads + 127) / 128); }
+
+void cpdf1d_points(const double* tt, long long n, const double* xs, int npts, int exact, double fz,
+                   const PdfChunks& k, double* part, double* ys, const LaunchCfg& c)
 {
     if (npts <= 0) return;
-    ++g_launches;
-    k_rel2d_points<<<dim3((npts + 63) / 64, nch), 64, 0, c.stream>>>(tt, kidx, nk, CC, full, chunk, xs, ys, npts,
-                                                                      part, bad);
+    g_launches += 2;
+    k_cpdf1d_points<<<pdf_blocks((long long)npts * k.nch), 128, 0, c.stream>>>(tt, n, xs, npts, exact, k.chunk, k.nch,
+                                                                              part);
+    k_pdf_finish<<<pdf_blocks((long long)npts * 32), 128, 0, c.stream>>>(part, k.nch, npts, exact, kTwoPiInv, 1.0, 1.0,
+                                                                        fz, ys);
+}
+
+void cpdf2d_points(const double* tt, long long n, int MC, const double* xs, const double* ys, int npts, double fz,
+                   const PdfChunks& k, double* part, double* zs, int* bad, const LaunchCfg& c)
+{
+    if (npts <= 0) return;
+    g_launches += 2;
+    k_cpdf2d_points<<<pdf_blocks((long long)npts * k.nch), 128, 0, c.stream>>>(
+        tt, nullptr, n, cpdf2d_stride(MC), 1, xs, ys, npts, k.chunk, k.nch, part, bad);
+    k_pdf_finish<<<pdf_blocks((long long)npts * 32), 128, 0, c.stream>>>(part, k.nch, npts, 0, 0.0, 2.0, kTwoPiInv, fz,
+                                                                        zs);
+}
+
+// Relative 2-D pdf (eval_marg2d_relative_and_transformed_cpdf,
+// cauchy_prediction.hpp:973-1073) over the kept pairs: the integral of a cell
+// is the marginal 2-D one.
+void rel2d_points(const double* tt, const long long* kidx, long long nk, int CC, int full, const double* xs,
+                  const double* ys, int npts, double nf, const PdfChunks& k, double* part, double* zs, int* bad,
+                  const LaunchCfg& c)
+{
+    if (npts <= 0) return;
+    g_launches += 2;
+    k_cpdf2d_points<<<pdf_blocks((long long)npts * k.nch), 128, 0, c.stream>>>(
+        tt, kidx, nk, rel2d_stride(CC), 1 + full, xs, ys, npts, k.chunk, k.nch, part, bad);
+    k_pdf_finish<<<pdf_blocks((long long)npts * 32), 128, 0, c.stream>>>(part, k.nch, npts, 0, 0.0, (double)(2 - full),
+                                                                        kTwoPiInv, nf, zs);
 }
 
 // kidx[kpos[j]] = j for every kept pair j (kpos: exclusive scan of keep)
@@ -3683,14 +3714,6 @@ void rel2d_compact(const int* keep, const long long* kpos, long long n, long lon
     if (n <= 0) return;
     ++g_launches;
     k_rel2d_compact<<<grid_for(n, 256, c.num_sms, 8), 256, 0, c.stream>>>(keep, kpos, n, kidx);
-}
-
-void rel2d_finish(const double* part, int nch, int npts, int full, double nf_prim, double nf_sec, double* zs,
-                  const LaunchCfg& c)
-{
-    if (npts <= 0) return;
-    ++g_launches;
-    k_rel2d_finish<<<(npts + 127) / 128, 128, 0, c.stream>>>(part, nch, npts, full, nf_prim, nf_sec, zs);
 }
 
 // Relative moments: a thread per (chunk, column) sums its chunk of pairs in

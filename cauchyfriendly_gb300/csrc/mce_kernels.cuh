@@ -138,8 +138,10 @@ struct Rel2DArgs {
     int* keep;              // npairs: 0 where the term was approximated out
     double* mrows;          // npairs x 14: g, g y_j, -(g y_j y_k) as (re, im)
 };
-// doubles per cache row: m, b[2], sin[CC+1], cos[CC+1], gamma1 re[CC], gamma2 re[CC], g[CC] (re, im)
-__host__ __device__ inline int rel2d_stride(int CC) { return 6 * CC + 5; }
+// doubles per record of a 2-D term of at most C cells: m, b[2], per cell its
+// first wall's sine and cosine, gamma1 re, gamma2 re, g (re, im); the last wall
+__host__ __device__ inline int marg2d_stride(int C) { return 6 * C + 5; }
+__host__ __device__ inline int rel2d_stride(int CC) { return marg2d_stride(CC); }
 
 // bucket positions kept per record between term-reduction rounds
 constexpr int kFtrResume = 8;
@@ -258,23 +260,28 @@ struct Kernels {
 
 // Shape-agnostic kernels.
 void group_count(const int* status, const int* owner, long long nR, int* gcnt, const LaunchCfg& c);
+// The pdf grids' split of n terms over npts points: nch chunks of `chunk`
+// terms per point, their sums in part[nch * npts].
+struct PdfChunks {
+    long long chunk = 1;
+    int nch = 1;
+};
+PdfChunks pdf_chunks(long long n, int npts, int waves, const LaunchCfg& c);
 // doubles per term record of the marginal 2-D pdf
-__host__ __device__ inline int cpdf2d_stride(int MC) { return 6 * MC + 6; }
+__host__ __device__ inline int cpdf2d_stride(int MC) { return marg2d_stride(MC); }
 // marginal 2-D pdf at npts points (xs, ys) from the per-term records of k_cpdf2d_terms
 void cpdf2d_points(const double* tt, long long n, int MC, const double* xs, const double* ys, int npts, double fz,
-                   double* zs, int* bad, const LaunchCfg& c);
+                   const PdfChunks& k, double* part, double* zs, int* bad, const LaunchCfg& c);
 // marginal 1-D pdf at npts points from the per-term records of k_cpdf1d_terms
-void cpdf1d_points(const double* tt, long long n, const double* xs, int npts, int exact, double fz, double* ys,
-                   const LaunchCfg& c);
-// relative 2-D pdf at npts points from the cache rows of the nk kept pairs
-// kidx (in order), split into nch chunks: part[nch x npts], then the chunk
-// sums in order scaled by (2 - full) (1/2pi)^2 / (nf_prim nf_sec)
-void rel2d_points(const double* tt, const long long* kidx, long long nk, int CC, int full, long long chunk,
-                  int nch, const double* xs, const double* ys, int npts, double* part, int* bad, const LaunchCfg& c);
+void cpdf1d_points(const double* tt, long long n, const double* xs, int npts, int exact, double fz,
+                   const PdfChunks& k, double* part, double* ys, const LaunchCfg& c);
+// relative 2-D pdf at npts points from the records of the nk kept pairs kidx
+// (in order), scaled by (2 - full) (1/2pi)^2 / nf
+void rel2d_points(const double* tt, const long long* kidx, long long nk, int CC, int full, const double* xs,
+                  const double* ys, int npts, double nf, const PdfChunks& k, double* part, double* zs, int* bad,
+                  const LaunchCfg& c);
 // kept pair indices in order from the keep flags and their exclusive scan
 void rel2d_compact(const int* keep, const long long* kpos, long long n, long long* kidx, const LaunchCfg& c);
-void rel2d_finish(const double* part, int nch, int npts, int full, double nf_prim, double nf_sec, double* zs,
-                  const LaunchCfg& c);
 // relative moments: the 14 columns of mrows summed over the pairs in order
 // (chunks of `chunk` pairs, then the chunk sums), finalised into out[14]
 void rel2d_moments(const double* mrows, long long n, long long chunk, double* part, double* out, const LaunchCfg& c);

@@ -240,3 +240,29 @@ def test_gpu_nd_pdf_against_oracle_on_larger_estimators():
     with pytest.raises(_lib.MceError):
         est.cpdf_nd(np.zeros(4))
     est.close()
+
+
+@pytest.mark.parametrize("updates,nx,ny", [(1, 2, 2), (2, 31, 3), (4, 33, 40), (6, 1030, 5)])
+def test_gpu_pdf_grids_do_not_depend_on_how_the_terms_are_split(updates, nx, ny):
+    """The grids' terms are summed in chunks whose number depends on the
+    points: 2 to 5,150 points of 3 to some hundred terms against the oracle's
+    term-by-term sums, within REL_TOL."""
+    _, CE, _ = _need_gpu()
+    from cauchyfriendly_gb300 import workloads as W
+    prob = W.two_state_lti(seed=4, steps=8)
+    rp, bp = oracle.draw_reference_constants(77, 2, oracle.max_shape_of(prob))
+    orc = oracle.Oracle(prob, rp, bp)
+    est = CE(prob["A0"], prob["p0"], prob["b0"], prob["steps"], 2, 0, 1, 1, root_point=rp, b_pert=bp)
+    for k in range(updates):
+        orc.step(k)
+        est.step(prob["msmts"][k, 0], prob["Phi"], prob["Gamma"], prob["beta"], prob["H"][0], prob["gamma"][0])
+    nu = np.array([0.7, 1.3])
+    gx, gy = (-1.0, 1.0, 2.0 / (nx - 1.5)), (-0.5, 0.5, 1.0 / (ny - 1.5))
+    xg, yg = est.cpdf_1d_grid(0, 0, *gx, nu)
+    xo, yo = orc.cpdf_1d_grid(0, nu, *gx)
+    assert len(xg) == nx and np.array_equal(xg, xo) and G.relerr(yg, yo) <= G.REL_TOL
+    X, Y, Z = est.cpdf_2d_grid(0, 0, 1, gx, gy, nu)
+    Xo, Yo, Zo = orc.cpdf_2d_grid(0, 1, nu, gx, gy, reset_cache=True)
+    assert len(X) == nx * ny and np.array_equal(X, Xo.reshape(-1)) and np.array_equal(Y, Yo.reshape(-1))
+    assert G.relerr(Z, Zo.reshape(-1)) <= G.REL_TOL
+    est.close()
