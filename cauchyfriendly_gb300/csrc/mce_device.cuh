@@ -53,6 +53,12 @@ __device__ inline cd cmul(cd x, cd y)
     double ac = x.re * y.re, bd = x.im * y.im, ad = x.re * y.im, bc = x.im * y.re;
     return cd{ac - bd, ad + bc};
 }
+// The product with its four real products on the integer pipe.
+__device__ inline cd cmul_i(cd x, cd y)
+{
+    const double ac = imul(x.re, y.re), bd = imul(x.im, y.im), ad = imul(x.re, y.im), bc = imul(x.im, y.re);
+    return cd{ac - bd, ad + bc};
+}
 __device__ inline unsigned long long dabs_bits(double x);
 
 // Complex division by R. L. Smith, "Algorithm 116: Complex division",
@@ -70,11 +76,11 @@ __device__ inline cd cdiv(cd x, cd y)
     const double p = big_c ? c : d, q = big_c ? d : c;
     const double P = big_c ? a : b, Q = big_c ? b : a;
     const double r = divide(q, p);
-    const double den = q * r + p;
-    const double pr = P * r;
+    const double den = imul(q, r) + p;
+    const double pr = imul(P, r);
     const double num = big_c ? (Q - pr) : (pr - Q);
     const DivBy by = div_by(den);
-    return cd{divide(Q * r + P, by), divide(num, by)};
+    return cd{divide(imul(Q, r) + P, by), divide(num, by)};
 }
 
 // Comparisons of doubles on their bit patterns (integer pipe).  IEEE doubles
@@ -191,10 +197,28 @@ __host__ __device__ inline int half_cells_cap(int m, int d)
     return c < 1 ? 1 : c;
 }
 
+// x in single precision, truncated (values of |x| < 2^127; below 2^-126: 0).
+__device__ inline float trunc32(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x);
+    int h = (int)(hi & 0x7fffffffu) - (896 << 20);  // the exponent's bias, 1023 to 127
+    h = h > 0 ? h : 0;
+    const unsigned f = __funnelshift_l((unsigned)__double2loint(x), (unsigned)h, 3);
+    return __uint_as_float(f | (hi & 0x80000000u));
+}
+
 // Row-vs-row coalignment gate (cauchy_term.hpp:494-504): +1 same, -1 opposite, 0 none.
+// The rows are normalised (entries of at most one), so single-precision first
+// entries that differ, and do not cancel, by more than 3e-7 (twice their
+// truncation, with room for the gate's 1e-8) settle nearly every pair without
+// the FP64 pipe.
 template <int D>
 __device__ inline int coalign_gate(const double* r, const double* c)
 {
+    {
+        const float a = trunc32(r[0]), b = trunc32(c[0]);
+        if (fabsf(a - b) > 3e-7f && fabsf(a + b) > 3e-7f) return 0;
+    }
     bool ps = true, ng = true;
 #pragma unroll
     for (int l = 0; l < D; l++) {
@@ -222,6 +246,16 @@ __device__ inline int orientation_mask(const double* Ai, const double* Aj, int m
 // ---------------------------------------------------------------------------
 // Dense D x D linear algebra in the reference's operation order
 // (cauchy_linalg.hpp:1180-1390).
+
+// A product of the unrolled elimination and solves: on the integer pipe up to
+// D = 3, whose code still fits the instruction cache (k_build_B_vertices<3> in
+// the 331-estimator batch's last update 599 -> 483 us; with D = 5 the same
+// products took a 5-state window's 71 ms to 94).
+template <int D>
+__device__ inline double lu_mul(double a, double b)
+{
+    return D <= 3 ? imul(a, b) : a * b;
+}
 // Every index is a compile-time one (row exchanges are selects), so the
 // matrix stays in registers.  The exchanges are applied to b as well, and
 // perm[i] receives the row of the matrix that ends at row i.  piv receives
@@ -265,7 +299,7 @@ __device__ inline bool plu(double* A, double* b, int* perm, DivBy* piv)
             const double t = divide(A[k * D + j], piv[j]);
             A[k * D + j] = t;
 #pragma unroll
-            for (int q = j + 1; q < D; q++) A[k * D + q] -= t * A[j * D + q];
+            for (int q = j + 1; q < D; q++) A[k * D + q] -= lu_mul<D>(t, A[j * D + q]);
         }
     }
     return true;
@@ -278,16 +312,26 @@ __device__ inline void lu_solve_inplace(const double* LU, const DivBy* piv, doub
     for (int i = 0; i < D; i++) {
         double s = x[i];
 #pragma unroll
-        for (int j = 0; j < i; j++) s -= LU[i * D + j] * x[j];
+        for (int j = 0; j < i; j++) s -= lu_mul<D>(LU[i * D + j], x[j]);
         x[i] = s;
     }
 #pragma unroll
     for (int i = D - 1; i >= 0; i--) {
         double s = x[i];
 #pragma unroll
-        for (int j = D - 1; j > i; j--) s -= LU[i * D + j] * x[j];
+        for (int j = D - 1; j > i; j--) s -= lu_mul<D>(LU[i * D + j], x[j]);
         x[i] = divide(s, piv[i]);
     }
+}
+
+// |x| in single precision rounded down or up (up: by an ulp even where x is
+// exact), on the integer pipe: the FP64 pipe takes as long for a conversion as
+// for a product.
+__device__ inline float abs32(double x, bool up)
+{
+    const unsigned h = ((unsigned)__double2hiint(x) & 0x7fffffffu) - (896u << 20);
+    if (h - (1u << 20) >= (253u << 20)) return up ? __double2float_ru(fabs(x)) : __double2float_rd(fabs(x));
+    return __uint_as_float(__funnelshift_l((unsigned)__double2loint(x), h, 3) + (up ? 1u : 0u));
 }
 
 // Upper bound on the 1-norm of (LU)^-1 from packed factors with partial
@@ -301,7 +345,7 @@ __device__ inline float inv_norm1_bound(const double* LU)
 {
     float Ua[D * D];
     for (int i = 0; i < D; i++)
-        for (int j = i; j < D; j++) Ua[i * D + j] = fabsf(__double2float_ru(fabs(LU[i * D + j])));
+        for (int j = i; j < D; j++) Ua[i * D + j] = abs32(LU[i * D + j], true);
     float best = 0.f;
     for (int k = 0; k < D; k++) {
         float x[D];
@@ -310,7 +354,7 @@ __device__ inline float inv_norm1_bound(const double* LU)
             float acc = (i == k) ? 1.f : 0.f;
             for (int j = i + 1; j <= k; j++) acc += Ua[i * D + j] * x[j];
             // a lower bound of |u_ii| keeps the quotient an upper bound
-            const float den = __double2float_rd(fabs(LU[i * D + i]));
+            const float den = abs32(LU[i * D + i], false);
             x[i] = acc / den;
             colsum += x[i];
         }
@@ -333,7 +377,8 @@ template <int D>
 __device__ inline bool cond1_exceeds(const double* LU, const DivBy* piv, const int* perm, double nrm, double eps)
 {
     double inrm = -1;
-#pragma unroll
+    constexpr int kUnroll = D <= 3 ? D : 1;  // (as lu_mul: the instruction cache)
+#pragma unroll kUnroll
     for (int i = 0; i < D; i++) {
         double w[D];
 #pragma unroll

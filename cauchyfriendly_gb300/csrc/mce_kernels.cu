@@ -652,7 +652,7 @@ __global__ void k_build_B_vertices(ParentList P, long long nP, const long long* 
                 for (int q = 0; q < m - D; q++) {
                     while ((inmask >> a) & 1u) a++;
                     double s = 0.0;
-                    for (int j = 0; j < D; j++) s += As[a * D + j] * v[j];
+                    for (int j = 0; j < D; j++) s += lu_mul<D>(As[a * D + j], v[j]);
                     if (neg(s - bp[a])) niv |= 1 << a;
                     a++;
                 }
@@ -1002,7 +1002,7 @@ __global__ void __launch_bounds__(128) k_mu_terms(ParentList P, long long nP, co
             const bool sgp = pos(s);
             if (!sgp) sneg |= 1 << l;
             const double sc = sgp ? pl : -pl;  // p_l * sign, exact
-            for (int j = 0; j < D; j++) ty[j] += sc * row[j];
+            for (int j = 0; j < D; j++) ty[j] += imul(sc, row[j]);
             if (!(hof & (1u << l))) ygi += sc;
             for (int j = 0; j < D; j++) At[l * D + j] = row[j];
             pt[l] = pl;
@@ -1040,9 +1040,9 @@ __global__ void __launch_bounds__(128) k_mu_terms(ParentList P, long long nP, co
         put(0, g);
         for (int j = 0; j < D; j++) {
             const cd y = mkcd(-ty[j], bt[j]);
-            const cd gy = cmul(g, y);
+            const cd gy = cmul_i(g, y);
             put(1 + j, gy);
-            for (int kk = 0; kk < D; kk++) put(1 + D + j * D + kk, cmul(gy, mkcd(-ty[kk], bt[kk])));
+            for (int kk = 0; kk < D; kk++) put(1 + D + j * D + kk, cmul_i(gy, mkcd(-ty[kk], bt[kk])));
         }
         const long long pslot = i + P.kscan[pstart[e]];            // parent's record
         const long long cslot0 = pstart[e + 1] + P.kscan[i];       // first child's record
@@ -3559,10 +3559,12 @@ __device__ inline cd rdiv(double x, cd y)
     const bool big_c = !(dabs_bits(c) < dabs_bits(d));
     const double p = big_c ? c : d, q = big_c ? d : c;
     const double r = divide(q, p);
-    const DivBy by = div_by(q * r + p);
-    const double u = divide(x, by), v = divide(x * r, by);
+    const DivBy by = div_by(imul(q, r) + p);
+    const double u = divide(x, by), v = divide(imul(x, r), by);
     return big_c ? cd{u, -v} : cd{v, -u};
 }
+
+__device__ inline cd cscale_i(cd a, double s) { return cd{imul(a.re, s), imul(a.im, s)}; }
 
 // One cell's integral (marg2d_eval_term_for_cpdf / marg2d_cached_eval_term_for_cpdf,
 // cpdf_ndim.hpp:1602-1640, 1710-1740): the fast form, or, with gamma1 ~ 0,
@@ -3587,8 +3589,8 @@ __device__ inline double marg2d_cell(double s1, double c1, double s2, double c2,
     if (fast) {
         gamma2 = cmul(gamma2, gamma1);
         gamma1 = cmul(gamma1, gamma1);
-        const cd lo = rdiv(s1, cadd(cscale(gamma1, c1), cscale(gamma2, s1)));
-        const cd hi = rdiv(s2, cadd(cscale(gamma1, c2), cscale(gamma2, s2)));
+        const cd lo = rdiv(s1, cadd(cscale_i(gamma1, c1), cscale_i(gamma2, s1)));
+        const cd hi = rdiv(s2, cadd(cscale_i(gamma1, c2), cscale_i(gamma2, s2)));
         cell = cmul(csub(hi, lo), g);
     } else {
         const cd lo = cdiv(csub(cscale(gamma1, s1), cscale(gamma2, c1)), cadd(cscale(gamma1, c1), cscale(gamma2, s1)));

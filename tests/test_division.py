@@ -1,7 +1,8 @@
-"""The kernels' integer-pipe division (csrc/mce_div.cuh) compiled for the
-host: the same bits as IEEE division for seeds an ulp either side of the
-correctly rounded single-precision reciprocal (the hardware's is within one),
-over random operands and the edges where a digit or the rounding can go wrong."""
+"""The kernels' integer-pipe division and product (csrc/mce_div.cuh) compiled
+for the host: the same bits as IEEE's, the division for seeds an ulp either
+side of the correctly rounded single-precision reciprocal (the hardware's is
+within one), over random operands and the edges where a digit or the rounding
+can go wrong."""
 import ctypes
 import os
 import subprocess
@@ -16,6 +17,10 @@ SRC = """
 extern "C" void quotients(long n, const double* a, const double* b, double* q)
 {
     for (long i = 0; i < n; i++) q[i] = mce::divide(a[i], b[i]);
+}
+extern "C" void products(long n, const double* a, const double* b, double* q)
+{
+    for (long i = 0; i < n; i++) q[i] = mce::imul(a[i], b[i]);
 }
 """
 
@@ -37,12 +42,12 @@ def _operands(rng, n):
 
 
 @pytest.mark.parametrize("ulps", [-1, 0, 1])
-def test_quotients_are_the_ieee_quotients(tmp_path, ulps):
+def test_quotients_and_products_are_the_ieee_ones(tmp_path, ulps):
     src, lib = tmp_path / "q.cpp", tmp_path / "q.so"
     src.write_text(SRC)
     subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-ffp-contract=off", "-I" + CSRC,
                     "-DMCE_DIV_SEED_ULPS=(%d)" % ulps, str(src), "-o", str(lib)], check=True)
-    f = ctypes.CDLL(str(lib)).quotients
+    L = ctypes.CDLL(str(lib))
     rng = np.random.Generator(np.random.PCG64(5))
     n = 1_000_000
     a, b = _operands(rng, n), _operands(rng, n)
@@ -51,9 +56,11 @@ def test_quotients_are_the_ieee_quotients(tmp_path, ulps):
         t = (b[: n // 4] * _operands(rng, n // 4)).view(np.uint64) + rng.integers(0, 5, n // 4, dtype=np.uint64)
         a[: n // 4] = (t - np.uint64(2)).view(np.float64)
         want = a / b
-    got = np.zeros(n)
+        prod = a * b
     dp = ctypes.POINTER(ctypes.c_double)
-    f(ctypes.c_long(n), a.ctypes.data_as(dp), b.ctypes.data_as(dp), got.ctypes.data_as(dp))
-    nan = np.isnan(want)
-    assert np.array_equal(np.isnan(got), nan)
-    assert np.array_equal(got.view(np.uint64)[~nan], want.view(np.uint64)[~nan])
+    for f, want in ((L.quotients, want), (L.products, prod)):
+        got = np.zeros(n)
+        f(ctypes.c_long(n), a.ctypes.data_as(dp), b.ctypes.data_as(dp), got.ctypes.data_as(dp))
+        nan = np.isnan(want)
+        assert np.array_equal(np.isnan(got), nan)
+        assert np.array_equal(got.view(np.uint64)[~nan], want.view(np.uint64)[~nan])
