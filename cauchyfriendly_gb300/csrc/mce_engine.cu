@@ -54,6 +54,121 @@ static void set_error(const std::string& s) { g_last_error = s; }
         }                                                                                  \
     } while (0)
 
+// Device memory of the handles' buffers.  A handle's hundred-odd buffers grow
+// with its terms, and cudaMalloc / cudaFree (which wait for the whole device)
+// took a third of a sliding-window pass: 36 of 101 ms for 16 steps of a 4-state
+// manager, 126 of 335 ms for a 5-state one.  The buffers come from a
+// stream-ordered pool of the library, one per device, which keeps at most a
+// 32nd of the device's memory between uses (the driver returns what is above
+// that at the next synchronisation), and kPoolKeepIdle bytes once no handle is
+// alive.  Inside a step (AllocOn) buffers are freed and allocated in the order
+// of the handle's stream, on which all of a step's work is queued or joined;
+// elsewhere an allocation is complete, and a freed buffer's work done, before
+// the call returns, as with cudaMalloc and cudaFree.
+constexpr size_t kPoolKeepIdle = 256u << 20;
+extern thread_local cudaStream_t t_alloc_stream;  // of the step this thread is in, or null
+extern thread_local bool t_alloc_idle;            // the buffers being freed have no work left
+cudaError_t dev_malloc(void** p, size_t bytes);
+void dev_free(void* p);
+void pool_handles(int change);  // a handle was made (+1) or destroyed (-1)
+struct AllocOn {
+    cudaStream_t prev;
+    explicit AllocOn(cudaStream_t s) : prev(t_alloc_stream) { t_alloc_stream = s; }
+    ~AllocOn() { t_alloc_stream = prev; }
+};
+struct AllocIdle {
+    bool prev = t_alloc_idle;
+    AllocIdle() { t_alloc_idle = true; }
+    ~AllocIdle() { t_alloc_idle = prev; }
+};
+#if MCE_ONLY_DIM <= 0
+thread_local cudaStream_t t_alloc_stream = nullptr;
+thread_local bool t_alloc_idle = false;
+namespace {
+struct DevPool {
+    cudaMemPool_t pool = nullptr;   // null: plain cudaMalloc
+    cudaStream_t stream = nullptr;  // allocations outside a step
+};
+constexpr int kMaxDevices = 64;
+std::mutex g_pool_mu;
+DevPool* g_pools[kMaxDevices] = {};
+int g_pool_handles = 0;
+
+DevPool* device_pool()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (g_pools[dev]) return g_pools[dev];
+    DevPool* d = new DevPool();
+    cudaMemPoolProps pr;
+    memset(&pr, 0, sizeof(pr));
+    pr.allocType = cudaMemAllocationTypePinned;
+    pr.location.type = cudaMemLocationTypeDevice;
+    pr.location.id = dev;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemPoolCreate(&d->pool, &pr) == cudaSuccess) {
+        cudaMemGetInfo(&free_b, &total_b);
+        unsigned long long keep = total_b / 32;
+        if (cudaMemPoolSetAttribute(d->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking) != cudaSuccess) {
+            cudaMemPoolDestroy(d->pool);
+            d->pool = nullptr;
+        }
+    } else {
+        d->pool = nullptr;
+    }
+    cudaGetLastError();
+    g_pools[dev] = d;
+    return d;
+}
+}  // namespace
+
+cudaError_t dev_malloc(void** p, size_t bytes)
+{
+    DevPool* d = device_pool();
+    if (!d || !d->pool) return cudaMalloc(p, bytes);
+    const cudaStream_t st = t_alloc_stream ? t_alloc_stream : d->stream;
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
+    if (e != cudaSuccess) {
+        // what the pool keeps unused may be what is missing
+        cudaGetLastError();
+        cudaDeviceSynchronize();
+        cudaMemPoolTrimTo(d->pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, d->pool, st);
+    }
+    if (e == cudaSuccess && !t_alloc_stream) e = cudaStreamSynchronize(st);
+    return e;
+}
+
+void dev_free(void* p)
+{
+    DevPool* d = device_pool();
+    if (!d || !d->pool) {
+        cudaFree(p);
+        return;
+    }
+    if (t_alloc_stream) {
+        cudaFreeAsync(p, t_alloc_stream);
+        return;
+    }
+    if (!t_alloc_idle) cudaDeviceSynchronize();
+    cudaFree(p);  // (of pool memory: no synchronisation of its own)
+}
+
+void pool_handles(int change)
+{
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    g_pool_handles += change;
+    if (g_pool_handles > 0) return;
+    for (DevPool* d : g_pools)
+        if (d && d->pool) cudaMemPoolTrimTo(d->pool, kPoolKeepIdle);
+}
+#endif
+
 // Grow-only device buffer.
 template <typename T>
 struct DevBuf {
@@ -62,7 +177,7 @@ struct DevBuf {
     ~DevBuf() { release(); }
     void release()
     {
-        if (ptr) cudaFree(ptr);
+        if (ptr) dev_free(ptr);
         ptr = nullptr;
         cap = 0;
     }
@@ -77,15 +192,15 @@ struct DevBuf {
         }
         size_t want = std::max<size_t>(n, cap + cap / 2);
         want = std::max<size_t>(want, 64);
-        if (ptr) cudaFree(ptr);
-        ptr = nullptr;
-        cap = 0;
-        cudaError_t e = cudaMalloc(&ptr, want * sizeof(T));
+        release();
+        void* q = nullptr;
+        const cudaError_t e = dev_malloc(&q, want * sizeof(T));
         if (e != cudaSuccess) {
             cudaGetLastError();
             set_error("cudaMalloc of " + std::to_string(want * sizeof(T)) + " bytes failed: " + cudaGetErrorString(e));
             return MCE_ERR_NOMEM;
         }
+        ptr = static_cast<T*>(q);
         cap = want;
         return MCE_OK;
     }
@@ -814,6 +929,8 @@ public:
     {
         if (master_step != 0) return MCE_ERR_ARG;
         if (min_bytes > 0 && trim_pass(false) < min_bytes) return 0;
+        drain();
+        const AllocIdle idle;
         return trim_pass(true);
     }
     // the bytes the term-sized buffers hold; released when `release`
@@ -937,6 +1054,7 @@ public:
     {
         using clk = std::chrono::steady_clock;
         const auto t0 = clk::now();
+        const AllocOn alloc_on(lc.stream);
         const int ms = master_step;
         const int sub = ms % p;
         const bool with_tp = sub == 0;
@@ -2563,6 +2681,7 @@ mce_handle* mce_batch_create(int n_est, int d, int cmcc, int pncc, int p, const 
         return nullptr;
     }
     h = new mce_handle{eng};
+    pool_handles(1);
     if (status) *status = MCE_OK;
     return h;
 }
@@ -2789,7 +2908,11 @@ long long mce_rel2d_num_pairs(mce_rel2d* r) { return r ? r->npairs : MCE_ERR_ARG
 long long mce_rel2d_num_terms(mce_rel2d* r) { return r ? r->nkept : MCE_ERR_ARG; }
 double mce_rel2d_device_ms(mce_rel2d* r, int which) { return r && which >= 0 && which < 3 ? r->ms[which] : -1.0; }
 long long mce_rel2d_launch_count(mce_rel2d* r) { return r ? r->launches : MCE_ERR_ARG; }
-void mce_rel2d_destroy(mce_rel2d* r) { delete r; }
+void mce_rel2d_destroy(mce_rel2d* r)
+{
+    const AllocIdle idle;  // the destructor waits for the object's stream first
+    delete r;
+}
 long long mce_post_mu_terms(mce_handle* h) { return h ? h->eng->post_mu_terms : MCE_ERR_ARG; }
 double mce_host_time_ms(mce_handle* h, int which) { return h && which >= 0 && which < 3 ? h->eng->host_ms[which] : -1.0; }
 int mce_master_step(mce_handle* h) { return h ? h->eng->master_step : MCE_ERR_ARG; }
@@ -2892,8 +3015,13 @@ const char* mce_autotune_kernel_name(int k)
 void mce_destroy(mce_handle* h)
 {
     if (!h) return;
-    delete h->eng;
-    delete h;
+    {
+        // the engine's destructor waits for its streams before its buffers go
+        const AllocIdle idle;
+        delete h->eng;
+        delete h;
+    }
+    pool_handles(-1);
 }
 
 }  // extern "C"
