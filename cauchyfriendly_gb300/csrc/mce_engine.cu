@@ -681,16 +681,17 @@ public:
     DevBuf<int> mu_ints;
     DevBuf<long long> goff, toff, rscan, bucket_off, rbase, scan_tmp, kall_est, ptile_start;
     DevBuf<int> status, owner, gcnt, gfill, members, members_tmp, is_root, cap, roots_list, alive, src,
-        tcnt, hist, new_slot, counters, first_cnt, bcount, bfill, slot_of, ptile_n, ptile_c;
+        tcnt, hist, new_slot, counters, first_cnt, bcount, slot_of, ptile_n, ptile_c;
     DevBuf<long long> boff;
     DevBuf<unsigned char> cell_ent, cell_ent2;
-    // number of bucket entries (valid records), known after the bucket scan
-    long long nvalid_entries(long long H) { return read_ll(boff.ptr + H); }
     // raw moments and G_SCALE_FACTOR per estimator, read back asynchronously
     // at the join and used after the step's final synchronisation
     PinnedBuf<cd> h_raw;
     PinnedBuf<double> h_gscale;
-    std::vector<int> h_hist;
+    // totals and counts a step reads back, written by its kernels or copied
+    // without a detour over pageable memory
+    PinnedBuf<long long> h_tot;
+    PinnedBuf<int> h_ints, h_hist;
     ScanScratch ss{};
     // profiling events
     std::vector<cudaEvent_t> evpool;
@@ -836,6 +837,9 @@ public:
         s |= scan_tmp.ensure(1 << 16);
         s |= h_raw.ensure((size_t)E * (1 + D + D * D));
         s |= h_gscale.ensure(E);
+        s |= h_tot.ensure(16);
+        s |= h_ints.ensure(8);
+        s |= h_hist.ensure((size_t)E * (MC + 1));
         if (s) return MCE_ERR_NOMEM;
         ss.block_sums = scan_tmp.ptr;
         ss.cap = (long long)scan_tmp.cap;
@@ -950,7 +954,7 @@ public:
         rel(Rb.horthog), rel(Rb.A), rel(Rb.p), rel(Rb.q), rel(Rb.b), rel(Rb.cval), rel(Rb.dval), rel(Rb.ps2);
         rel(Rb.cmap), rel(Rb.csmap);
         rel(Bcap), rel(Bkeys), rel(kall_scan), rel(nvert), rel(voff), rel(vsv), rel(fam_mom), rel(mu_rows);
-        rel(mu_ints), rel(bcount), rel(bfill), rel(boff), rel(slot_of), rel(cell_ent), rel(cell_ent2), rel(status);
+        rel(mu_ints), rel(bcount), rel(boff), rel(slot_of), rel(cell_ent), rel(cell_ent2), rel(status);
         rel(owner), rel(ftr_wl[0]), rel(ftr_wl[1]), rel(ftr_resume), rel(gcnt), rel(gfill), rel(goff), rel(members);
         rel(members_tmp), rel(is_root), rel(cap), rel(rscan), rel(toff), rel(roots_list), rel(alive), rel(src);
         rel(tcnt), rel(g_nr), rel(g_items), rel(g_cells), rel(g_ioff), rel(g_coff), rel(g_rps2), rel(g_rflag);
@@ -1029,24 +1033,16 @@ public:
     int sync_and_check()
     {
         MCE_CUDA(cudaGetLastError());
+        MCE_CUDA(cudaMemcpyAsync(h_ints.data() + 4, counters.ptr, sizeof(int), cudaMemcpyDeviceToHost, lc.stream));
         MCE_CUDA(cudaStreamSynchronize(lc.stream));
         if (ftr_graph) Kernels<D>::ftr_graph_collect(ftr_graph);
-        int err = 0;
-        MCE_CUDA(cudaMemcpy(&err, counters.ptr, sizeof(int), cudaMemcpyDeviceToHost));
+        const int err = h_ints[4];
         if (err) {
             device_errors |= err;
             set_error("device error bits " + std::to_string(err));
             return MCE_ERR_DEVICE;
         }
         return MCE_OK;
-    }
-
-    long long read_ll(const long long* p_)
-    {
-        long long v = 0;
-        cudaMemcpyAsync(&v, p_, sizeof(long long), cudaMemcpyDeviceToHost, lc.stream);
-        cudaStreamSynchronize(lc.stream);
-        return v;
     }
 
     int step(const double* msmt, const double* Phi, const double* Gamma, const double* beta, const double* H,
@@ -1313,18 +1309,15 @@ public:
         Kernels<D>::tp(PV, nP, dsteps.ptr, with_tp ? 1 : 0, MC, Bcap.ptr, nvert.ptr, err, lc);
         pend();
         pbeg(KID_SCAN);
-        scan_int_to_ll(PV.nkids, PV.kscan, nP, ss, lc);
-        scan_int_to_ll(Bcap.ptr, PV.B_off, nP, ss, lc);
-        scan_int_to_ll(PV.nkids_all, kall_scan.ptr, nP, ss, lc);
-        scan_int_to_ll(nvert.ptr, voff.ptr, nP, ss, lc);
+        long long* tot = h_tot.data();  // the kernels write the totals here
+        const ScanJob build_jobs[4] = {{PV.nkids, PV.kscan, tot},
+                                       {Bcap.ptr, PV.B_off, tot + 1},
+                                       {PV.nkids_all, kall_scan.ptr, tot + 2},
+                                       {nvert.ptr, voff.ptr, tot + 3}};
+        scan_many(build_jobs, 4, nP, ss, lc);
         pend();
-        long long tot[4] = {0, 0, 0, 0};
-        MCE_CUDA(cudaMemcpyAsync(&tot[0], PV.kscan + nP, sizeof(long long), cudaMemcpyDeviceToHost, lc.stream));
-        MCE_CUDA(cudaMemcpyAsync(&tot[1], PV.B_off + nP, sizeof(long long), cudaMemcpyDeviceToHost, lc.stream));
-        MCE_CUDA(cudaMemcpyAsync(&tot[2], kall_scan.ptr + nP, sizeof(long long), cudaMemcpyDeviceToHost, lc.stream));
-        MCE_CUDA(cudaMemcpyAsync(&tot[3], voff.ptr + nP, sizeof(long long), cudaMemcpyDeviceToHost, lc.stream));
         // per-estimator post-MU counts for the un-reduced final MU
-        std::vector<long long> kall_at(E + 1, 0);
+        std::vector<long long> kall_at;
         MCE_CUDA(cudaStreamSynchronize(lc.stream));
         const long long K = tot[0], Btot = tot[1], Kall = tot[2], Nvert = tot[3];
         const long long nR = nP + K;
@@ -1385,13 +1378,6 @@ public:
             pend(mstream);
         }
         MCE_CUDA(cudaEventRecord(ev_join, mstream));
-        // terms after the MU per estimator (un-reduced count, cauchy_estimator.hpp:749-751, 806-812)
-        if ((s = kall_est.ensure(E + 2))) return s;
-        pbeg(KID_SCAN);
-        k_gather_bounds(kall_scan.ptr, E);
-        pend();
-        MCE_CUDA(cudaMemcpyAsync(kall_at.data(), kall_est.ptr, sizeof(long long) * (E + 1), cudaMemcpyDeviceToHost,
-                                 lc.stream));
         // shapes of the final-MU estimators (terms_per_shape of the parents' shapes)
         std::vector<int> skip_hist;
         bool any_skip = false, any_keep = false;
@@ -1401,6 +1387,14 @@ public:
         }
         const int MCp = MC + 1;
         if (any_skip) {
+            // terms after the MU per estimator (un-reduced count, cauchy_estimator.hpp:749-751, 806-812)
+            if ((s = kall_est.ensure(E + 2))) return s;
+            pbeg(KID_SCAN);
+            k_gather_bounds(kall_scan.ptr, E);
+            pend();
+            kall_at.assign(E + 1, 0);
+            MCE_CUDA(cudaMemcpyAsync(kall_at.data(), kall_est.ptr, sizeof(long long) * (E + 1),
+                                     cudaMemcpyDeviceToHost, lc.stream));
             if ((s = hist.ensure((size_t)E * MCp))) return s;
             if (!any_keep) {
                 // every estimator ends its step here: the step waits for its
@@ -1417,9 +1411,9 @@ public:
             skip_hist.resize((size_t)E * MCp);
             MCE_CUDA(cudaMemcpyAsync(skip_hist.data(), hist.ptr, sizeof(int) * E * MCp, cudaMemcpyDeviceToHost,
                                      lc.stream));
+            MCE_CUDA(cudaStreamSynchronize(lc.stream));
         }
-        MCE_CUDA(cudaStreamSynchronize(lc.stream));
-        for (int e = 0; e < E; e++) {
+        for (int e = 0; any_skip && e < E; e++) {
             if (!hsteps[e].active) continue;
             if (hsteps[e].skip) {
                 est[e].nt = (hpstart[e + 1] - hpstart[e]) + (kall_at[e + 1] - kall_at[e]);
@@ -1439,29 +1433,31 @@ public:
         // ---- fast term reduction
         long long H = 1;
         while (H < nR) H <<= 1;
-        if ((s = bcount.ensure(H + 1))) return s;
-        if ((s = bfill.ensure(H + 1))) return s;
+        if ((s = bcount.ensure(2 * H + 2))) return s;  // the buckets' counts, then their fill counts
+        int* const bfill = bcount.ptr + H;
         if ((s = boff.ensure(H + 2))) return s;
         if ((s = slot_of.ensure(nR + 1))) return s;
         if ((s = cell_ent.ensure((nR + 1) * Kernels<D>::cell_entry_bytes()))) return s;
         if ((s = cell_ent2.ensure((nR + 1) * Kernels<D>::cell_entry_bytes()))) return s;
         if ((s = status.ensure(nR + 1))) return s;
         if ((s = owner.ensure(nR + 1))) return s;
+        if ((s = gcnt.ensure(nR + 1))) return s;
+        if ((s = gfill.ensure(nR + 1))) return s;
+        if ((s = ftr_cnt.ensure(kFtrCntSlots))) return s;
         if ((s = ensure_scan_scratch(std::max(nR, H) + 1))) return s;
-        MCE_CUDA(cudaMemsetAsync(bcount.ptr, 0, sizeof(int) * H, lc.stream));
-        MCE_CUDA(cudaMemsetAsync(bfill.ptr, 0, sizeof(int) * H, lc.stream));
+        MCE_CUDA(cudaMemsetAsync(bcount.ptr, 0, sizeof(int) * 2 * H, lc.stream));
         pbeg(KID_FTR);
-        Kernels<D>::ftr_cells(R, nR, H - 1, slot_of.ptr, bcount.ptr, lc);
+        Kernels<D>::ftr_cells(R, nR, H - 1, slot_of.ptr, bcount.ptr,
+                              FtrInit{status.ptr, gcnt.ptr, gfill.ptr, ftr_cnt.ptr, kFtrCntSlots}, lc);
         pend();
         pbeg(KID_SCAN);
         scan_int_to_ll(bcount.ptr, boff.ptr, H, ss, lc);
         pend();
-        const long long nent = nvalid_entries(H);  // bucket entries = valid records
         pbeg(KID_FTR);
-        Kernels<D>::ftr_scatter(R, nR, slot_of.ptr, boff.ptr, bfill.ptr, cell_ent.ptr, lc);
+        Kernels<D>::ftr_scatter(R, nR, slot_of.ptr, boff.ptr, bfill, cell_ent.ptr, lc);
         // sort each bucket by term index
-        Kernels<D>::ftr_sort(cell_ent.ptr, nent, slot_of.ptr, boff.ptr, cell_ent2.ptr, lc);
-        k_status_init(R, nR);
+        // (boff's total: the valid records)
+        Kernels<D>::ftr_sort(cell_ent.ptr, nR, boff.ptr + H, slot_of.ptr, boff.ptr, cell_ent2.ptr, lc);
         pend();
         if ((s = ftr_wl[0].ensure(nR + 1))) return s;
         if ((s = ftr_wl[1].ensure(nR + 1))) return s;
@@ -1470,14 +1466,12 @@ public:
         // kFtrFirstBatch): a round reads the previous round's worklist length
         // on the device, a round after the last is empty, and the host reads
         // the count once per batch
-        if ((s = ftr_cnt.ensure(kFtrCntSlots))) return s;
         // the first round over every record as an ordinary (full-occupancy)
         // launch; the rounds after it as ftr_rounds_mode() says: queued in
         // batches, the host reading the worklist length once per batch; in one
         // persistent cooperative launch over the device worklists; or as a
         // device-side loop in a CUDA graph (neither of the last two has a host
         // round trip).  The no-allocation step runs the batched rounds.
-        MCE_CUDA(cudaMemsetAsync(ftr_cnt.ptr, 0, sizeof(int) * kFtrCntSlots, lc.stream));
         pbeg(KID_FTR);
         Kernels<D>::ftr_resolve(R, nR, cell_ent2.ptr, boff.ptr, H - 1, MC, status.ptr, owner.ptr, nullptr, nullptr,
                                 nR, ftr_wl[0].ptr, ftr_cnt.ptr, ftr_resume.ptr, lc);
@@ -1502,7 +1496,8 @@ public:
             }
         }
         pend();
-        int unk = 0;
+        int* const unk = h_ints.data();
+        *unk = 0;
         long long bound = nR;
         for (int round = 1; pst != MCE_OK;) {
             // the rounds after the first queued in batches (round r counts
@@ -1511,18 +1506,18 @@ public:
             pbeg(KID_FTR);
             for (int q = 0; q < K; q++, round++) {
                 int* n_out = ftr_cnt.ptr + round % kFtrCntSlots;
-                MCE_CUDA(cudaMemsetAsync(n_out, 0, sizeof(int), lc.stream));
+                if (round >= kFtrCntSlots) MCE_CUDA(cudaMemsetAsync(n_out, 0, sizeof(int), lc.stream));
                 Kernels<D>::ftr_resolve(R, nR, cell_ent2.ptr, boff.ptr, H - 1, MC, status.ptr, owner.ptr,
                                         round ? ftr_wl[(round - 1) & 1].ptr : nullptr,
                                         round ? ftr_cnt.ptr + (round - 1) % kFtrCntSlots : nullptr, bound,
                                         ftr_wl[round & 1].ptr, n_out, ftr_resume.ptr, lc);
             }
             pend();
-            MCE_CUDA(cudaMemcpyAsync(&unk, ftr_cnt.ptr + (round - 1) % kFtrCntSlots, sizeof(int),
+            MCE_CUDA(cudaMemcpyAsync(unk, ftr_cnt.ptr + (round - 1) % kFtrCntSlots, sizeof(int),
                                      cudaMemcpyDeviceToHost, lc.stream));
             MCE_CUDA(cudaStreamSynchronize(lc.stream));
-            if (unk == 0) break;
-            bound = unk;
+            if (*unk == 0) break;
+            bound = *unk;
             if (round > 100000) {
                 set_error("term reduction did not converge");
                 device_errors |= kErrResolveStalled;
@@ -1530,49 +1525,35 @@ public:
             }
         }
         // ---- reduction groups
-        if ((s = gcnt.ensure(nR + 1))) return s;
-        if ((s = gfill.ensure(nR + 1))) return s;
         if ((s = goff.ensure(nR + 2))) return s;
-        MCE_CUDA(cudaMemsetAsync(gcnt.ptr, 0, sizeof(int) * (nR + 1), lc.stream));
-        MCE_CUDA(cudaMemsetAsync(gfill.ptr, 0, sizeof(int) * (nR + 1), lc.stream));
+        if ((s = is_root.ensure(nR + 1))) return s;
+        if ((s = cap.ensure(nR + 1))) return s;
+        if ((s = rscan.ensure(nR + 2))) return s;
+        if ((s = toff.ensure(nR + 2))) return s;
+        if ((s = alive.ensure(nR + 1))) return s;
         pbeg(KID_GROUPS);
-        group_count(status.ptr, owner.ptr, nR, gcnt.ptr, lc);
-        scan_int_to_ll(gcnt.ptr, goff.ptr, nR, ss, lc);
+        group_count(status.ptr, owner.ptr, Rb.m.ptr, nR, D, gcnt.ptr, is_root.ptr, cap.ptr, alive.ptr, lc);
+        const ScanJob group_jobs[3] = {
+            {gcnt.ptr, goff.ptr, nullptr}, {is_root.ptr, rscan.ptr, tot + 4}, {cap.ptr, toff.ptr, tot + 5}};
+        scan_many(group_jobs, 3, nR, ss, lc);
         pend();
         // each record is a member of at most one group: nR bounds the
         // members, so their buffers are sized without reading the count back
         const long long nmembers = nR;
         if ((s = members.ensure(nmembers + 1))) return s;
         if ((s = members_tmp.ensure(nmembers + 1))) return s;
-        pbeg(KID_GROUPS);
-        group_fill(status.ptr, owner.ptr, nR, goff.ptr, gfill.ptr, members_tmp.ptr, lc);
-        group_sort(gcnt.ptr, goff.ptr, nR, members_tmp.ptr, members.ptr, lc);
-        pend();
-        if ((s = is_root.ensure(nR + 1))) return s;
-        if ((s = cap.ensure(nR + 1))) return s;
-        if ((s = rscan.ensure(nR + 2))) return s;
-        if ((s = toff.ensure(nR + 2))) return s;
-        pbeg(KID_GROUPS);
-        roots_flags(status.ptr, Rb.m.ptr, nR, D, is_root.ptr, cap.ptr, lc);
-        scan_int_to_ll(is_root.ptr, rscan.ptr, nR, ss, lc);
-        scan_int_to_ll(cap.ptr, toff.ptr, nR, ss, lc);
-        pend();
-        long long t2[2];
-        MCE_CUDA(cudaMemcpyAsync(&t2[0], rscan.ptr + nR, sizeof(long long), cudaMemcpyDeviceToHost, lc.stream));
-        MCE_CUDA(cudaMemcpyAsync(&t2[1], toff.ptr + nR, sizeof(long long), cudaMemcpyDeviceToHost, lc.stream));
         MCE_CUDA(cudaStreamSynchronize(lc.stream));
-        const long long nroots = t2[0], ttot = t2[1];
+        const long long nroots = tot[4], ttot = tot[5];
         if ((s = roots_list.ensure(nroots + 1))) return s;
         pbeg(KID_GROUPS);
-        mce::roots_list(is_root.ptr, rscan.ptr, nR, roots_list.ptr, lc);
+        group_fill(status.ptr, owner.ptr, nR, goff.ptr, gfill.ptr, members_tmp.ptr, rscan.ptr, roots_list.ptr, lc);
+        group_sort(gcnt.ptr, goff.ptr, nR, members_tmp.ptr, members.ptr, lc);
         pend();
         TBufs& Tn = Tb[cur ^ 1];
         if ((s = Tn.keys.ensure(ttot + 1))) return s;
         if ((s = Tn.vals.ensure(ttot + 1))) return s;
-        if ((s = alive.ensure(nR + 1))) return s;
         if ((s = src.ensure(nR + 1))) return s;
         if ((s = tcnt.ensure(nR + 1))) return s;
-        MCE_CUDA(cudaMemsetAsync(alive.ptr, 0, sizeof(int) * (nR + 1), lc.stream));
         // cells a group may hold: a central arrangement in general position
         // has at most half_cells_cap(m, d) half-cells; nearly degenerate
         // arrangements can yield more, found by the preparation below
@@ -1602,21 +1583,17 @@ public:
                  g_mflag.ptr, nullptr,       pr_root.ptr,   pr_mb.ptr,    pr_mcnt.ptr,  pr_cells.ptr,
                  pr_items.ptr, pr_moff.ptr,  pr_ioff.ptr,   pr_coff.ptr,  nullptr};
         Tables Tnv{Tn.keys.ptr, Tn.vals.ptr};
-        long long gt[2] = {0, 0};
         for (int attempt = 0;; attempt++) {
             MCE_CUDA(cudaMemsetAsync(g_over.ptr, 0, 2 * sizeof(int), lc.stream));
             pbeg(KID_GTABLE);
             Kernels<D>::gtable_prep(R, roots_list.ptr, nroots, gcnt.ptr, goff.ptr, members.ptr, PV, Told, Bkeys.ptr,
                                     toff.ptr, Tnv, gf, g_items.ptr, g_cells.ptr, MC, cap.ptr, g_over.ptr, lc);
-            scan_int_to_ll(g_items.ptr, g_ioff.ptr, nroots, ss, lc);
-            scan_int_to_ll(g_cells.ptr, g_coff.ptr, nroots, ss, lc);
+            const ScanJob item_jobs[2] = {{g_items.ptr, g_ioff.ptr, tot + 6}, {g_cells.ptr, g_coff.ptr, tot + 7}};
+            scan_many(item_jobs, 2, nroots, ss, lc);
             pend();
-            int ov[2] = {0, 0};
+            int* const ov = h_ints.data() + 2;
+            ov[0] = ov[1] = 0;
             if (nroots > 0) {
-                MCE_CUDA(cudaMemcpyAsync(&gt[0], g_ioff.ptr + nroots, sizeof(long long), cudaMemcpyDeviceToHost,
-                                         lc.stream));
-                MCE_CUDA(cudaMemcpyAsync(&gt[1], g_coff.ptr + nroots, sizeof(long long), cudaMemcpyDeviceToHost,
-                                         lc.stream));
                 MCE_CUDA(cudaMemcpyAsync(ov, g_over.ptr, 2 * sizeof(int), cudaMemcpyDeviceToHost, lc.stream));
                 MCE_CUDA(cudaStreamSynchronize(lc.stream));
             }
@@ -1656,7 +1633,7 @@ public:
             if ((s = scratch.ensure((size_t)max_warps * capR))) return s;
             gscr = scratch.ptr;
         }
-        const long long nitems = gt[0], ncells = gt[1];
+        const long long nitems = nroots > 0 ? tot[6] : 0, ncells = nroots > 0 ? tot[7] : 0;
         if ((s = g_vals.ensure(nitems + 1))) return s;
         gf.gv = g_vals.ptr;
         if ((s = join_moments())) return s;
@@ -1665,25 +1642,18 @@ public:
                                 gscale.ptr, toff.ptr, Tnv, gf, MC, lc);
         Kernels<D>::gtable_combine(R, roots_list.ptr, nroots, g_coff.ptr, ncells, gcnt.ptr, goff.ptr, members.ptr, PV,
                                    Told, Bkeys.ptr, toff.ptr, Tnv, tcnt.ptr, alive.ptr, src.ptr, gf, MC, lc);
-        MCE_CUDA(cudaMemsetAsync(pr_mcnt.ptr, 0, sizeof(int) * (nroots + 1), lc.stream));
-        MCE_CUDA(cudaMemsetAsync(pr_cells.ptr, 0, sizeof(int) * (nroots + 1), lc.stream));
-        MCE_CUDA(cudaMemsetAsync(pr_items.ptr, 0, sizeof(int) * (nroots + 1), lc.stream));
         Kernels<D>::gtable(R, roots_list.ptr, nroots, gcnt.ptr, goff.ptr, members.ptr, PV, Told, Bkeys.ptr, gscale.ptr,
                            toff.ptr, Tnv, tcnt.ptr, alive.ptr, src.ptr, gscr, capR, gf, MC, err, lc, gscr_warps);
         // members left after promotions: the promoted-root flat pass
-        scan_int_to_ll(pr_mcnt.ptr, pr_moff.ptr, nroots, ss, lc);
-        scan_int_to_ll(pr_items.ptr, pr_ioff.ptr, nroots, ss, lc);
-        scan_int_to_ll(pr_cells.ptr, pr_coff.ptr, nroots, ss, lc);
+        const ScanJob prom_jobs[3] = {{pr_mcnt.ptr, pr_moff.ptr, tot + 8},
+                                      {pr_items.ptr, pr_ioff.ptr, tot + 9},
+                                      {pr_cells.ptr, pr_coff.ptr, tot + 10}};
+        if (nroots > 0) scan_many(prom_jobs, 3, nroots, ss, lc);
         pend();
         long long pt[3] = {0, 0, 0};
         if (nroots > 0) {
-            MCE_CUDA(cudaMemcpyAsync(&pt[0], pr_moff.ptr + nroots, sizeof(long long), cudaMemcpyDeviceToHost,
-                                     lc.stream));
-            MCE_CUDA(cudaMemcpyAsync(&pt[1], pr_ioff.ptr + nroots, sizeof(long long), cudaMemcpyDeviceToHost,
-                                     lc.stream));
-            MCE_CUDA(cudaMemcpyAsync(&pt[2], pr_coff.ptr + nroots, sizeof(long long), cudaMemcpyDeviceToHost,
-                                     lc.stream));
             MCE_CUDA(cudaStreamSynchronize(lc.stream));
+            for (int k = 0; k < 3; k++) pt[k] = tot[8 + k];
         }
         if (pt[1] > 0) {
             if ((s = pr_gv.ensure(pt[1] + 1))) return s;
@@ -1711,7 +1681,6 @@ public:
         partition_rank(alive.ptr, Rb.m.ptr, rbase.ptr, E, MCp, nR, ptile_start.ptr, ptile_c.ptr, bucket_off.ptr,
                        new_slot.ptr, lc);
         pend();
-        h_hist.resize((size_t)E * MCp);
         MCE_CUDA(cudaMemcpyAsync(h_hist.data(), hist.ptr, sizeof(int) * E * MCp, cudaMemcpyDeviceToHost, lc.stream));
         MCE_CUDA(cudaStreamSynchronize(lc.stream));
         std::vector<long long> np(E + 1, 0);
@@ -1781,7 +1750,7 @@ public:
             t = (t + 2047) / 2048;
             need += t + 2;
         }
-        int s = scan_tmp.ensure(need + 64);
+        int s = scan_tmp.ensure(need * kScanJobs + 64);
         if (s) return s;
         ss.block_sums = scan_tmp.ptr;
         ss.cap = (long long)scan_tmp.cap;
@@ -1790,7 +1759,6 @@ public:
 
     void k_skip_hist(ParentList PV, long long n, int MCp);
     void k_gather_bounds(const long long* scan, int E_);
-    void k_status_init(TermRecs R, long long nR);
 
     // ---- extended-mode helpers (cauchy_estimator.hpp:1312-1394)
     DevBuf<double> ext_buf;
@@ -2309,21 +2277,6 @@ void Engine<D>::alg_stats(bool with_tp, long long nR, bool tables_built)
         kbytes[k] += h[2 * k];
         kflops[k] += h[2 * k + 1];
     }
-}
-
-static __global__ void k_status_init_kernel(const int* est, long long n, int* status)
-{
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x)
-        status[j] = est[j] < 0 ? -1 : 0;
-}
-
-template <int D>
-void Engine<D>::k_status_init(TermRecs R, long long nR)
-{
-    if (nR == 0) return;
-    ++g_launches;
-    k_status_init_kernel<<<(int)std::min<long long>((nR + 255) / 256, lc.num_sms * 16), 256, 0, lc.stream>>>(
-        R.est, nR, status.ptr);
 }
 
 // Per-dimension factories: each dimension's engine lives in its own unit.

@@ -322,26 +322,110 @@ static void scan_ll_inplace(long long* data, long long n, long long* scratch, lo
     k_write_total<<<1, 32, 0, c.stream>>>(data, n, ts, ntiles);
 }
 
+// Up to kScanJobs scans of n values each (out[n] and, when set, *total receive
+// the sum): a step's buffers come from a dozen such scans, mostly of a few
+// hundred to a few thousand values, where a launch costs more than the scan.
+// One launch up to a tile; two (tile sums, then each tile with the sums before
+// it) up to kScanDirectTiles tiles; above, the tile sums are scanned in between.
+struct ScanJobs {
+    ScanJob j[kScanJobs];
+};
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_small(ScanJobs js, long long n)
+{
+    const ScanJob J = js.j[blockIdx.x];
+    const long long base = (long long)threadIdx.x * kScanItems;
+    long long v[kScanItems], s = 0, tot;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        v[k] = base + k < n ? (long long)J.in[base + k] : 0;
+        s += v[k];
+    }
+    long long pre = block_exclusive_scan<long long>(s, &tot);
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        if (base + k < n) J.out[base + k] = pre;
+        pre += v[k];
+    }
+    if (threadIdx.x == 0) {
+        J.out[n] = tot;
+        if (J.total) *J.total = tot;
+    }
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(ScanJobs js, long long n, long long* sums, long long pitch)
+{
+    const int* in = js.j[blockIdx.y].in;
+    const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
+    long long s = 0, tot;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++)
+        if (base + k < n) s += in[base + k];
+    block_exclusive_scan<long long>(s, &tot);
+    if (threadIdx.x == 0) sums[blockIdx.y * pitch + blockIdx.x] = tot;
+}
+
+// scanned: the sums are exclusive offsets already
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(ScanJobs js, long long n, const long long* sums,
+                                                             long long pitch, int scanned)
+{
+    const ScanJob J = js.j[blockIdx.y];
+    sums += blockIdx.y * pitch;
+    long long before = 0, tot;
+    if (scanned) {
+        before = sums[blockIdx.x];
+    } else {
+        long long s = 0;
+        for (int k = threadIdx.x; k < (int)blockIdx.x; k += kScanThreads) s += sums[k];
+        block_exclusive_scan<long long>(s, &before);
+    }
+    const long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
+    long long v[kScanItems], s = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        v[k] = base + k < n ? (long long)J.in[base + k] : 0;
+        s += v[k];
+    }
+    long long pre = before + block_exclusive_scan<long long>(s, &tot);
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        if (base + k < n) J.out[base + k] = pre;
+        pre += v[k];
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        J.out[n] = before + tot;
+        if (J.total) *J.total = before + tot;
+    }
+}
+
+void scan_many(const ScanJob* jobs, int njobs, long long n, ScanScratch& s, const LaunchCfg& c)
+{
+    constexpr long long kScanDirectTiles = 1024;
+    ScanJobs js{};
+    for (int k = 0; k < njobs; k++) js.j[k] = jobs[k];
+    const long long ntiles = (n + kScanTile - 1) / kScanTile;
+    if (ntiles <= 1) {
+        ++g_launches;
+        k_scan_small<<<njobs, kScanThreads, 0, c.stream>>>(js, n);
+        return;
+    }
+    const dim3 grid((unsigned)ntiles, njobs);
+    const long long pitch = ntiles + 1;
+    long long* sums = s.block_sums;
+    ++g_launches;
+    k_scan_sums<<<grid, kScanThreads, 0, c.stream>>>(js, n, sums, pitch);
+    const bool scanned = ntiles > kScanDirectTiles;
+    if (scanned)
+        for (int k = 0; k < njobs; k++)
+            scan_ll_inplace(sums + k * pitch, ntiles, s.block_sums + njobs * pitch, s.cap - njobs * pitch, c);
+    ++g_launches;
+    k_scan_apply<<<grid, kScanThreads, 0, c.stream>>>(js, n, sums, pitch, scanned ? 1 : 0);
+}
+
 void scan_int_to_ll(const int* in, long long* out, long long n, ScanScratch& s, const LaunchCfg& c)
 {
-    const long long ntiles = (n + kScanTile - 1) / kScanTile;
-    if (n == 0) {
-        cudaMemsetAsync(out, 0, sizeof(long long), c.stream);
-        return;
-    }
-    long long* ts = s.block_sums;
-    ++g_launches;
-    k_scan_tiles<int><<<(unsigned)ntiles, kScanThreads, 0, c.stream>>>(in, out, n, ts);
-    if (ntiles == 1) {
-        ++g_launches;
-        k_copy_ll<<<1, 32, 0, c.stream>>>(ts, out + n, 1);
-        return;
-    }
-    scan_ll_inplace(ts, ntiles, s.block_sums + ntiles + 1, s.cap - (ntiles + 1), c);
-    ++g_launches;
-    k_scan_add<<<(unsigned)ntiles, kScanThreads, 0, c.stream>>>(out, n, ts);
-    ++g_launches;
-    k_write_total<<<1, 32, 0, c.stream>>>(out, n, ts, ntiles);
+    const ScanJob j{in, out, nullptr};
+    scan_many(&j, 1, n, s, c);
 }
 
 #endif  // MCE_COMMON_UNIT
@@ -1224,10 +1308,15 @@ struct CellEntry {
 };
 
 template <int D>
-__global__ void k_ftr_count_cells(TermRecs R, long long nR, long long hmask, int* slot_of, int* bcount)
+__global__ void k_ftr_count_cells(TermRecs R, long long nR, long long hmask, int* slot_of, int* bcount, FtrInit z)
 {
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < nR; j += (long long)gridDim.x * blockDim.x) {
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t0 < z.ncnt) z.cnt[t0] = 0;
+    for (long long j = t0; j < nR; j += (long long)gridDim.x * blockDim.x) {
         const int e = R.est[j];
+        z.status[j] = e < 0 ? -1 : 0;
+        z.gcnt[j] = 0;
+        z.gfill[j] = 0;
         if (e < 0) {
             slot_of[j] = -1;
             continue;
@@ -1281,9 +1370,10 @@ __device__ inline bool ftr_near_pm(const TermRecs& R, long long i, long long j, 
 
 // Buckets in ascending term order: every entry ranks itself inside its bucket.
 template <int D>
-__global__ void k_ftr_sort_buckets(const CellEntry<D>* in, long long n, const int* slot_of, const long long* boff,
-                                   CellEntry<D>* out)
+__global__ void k_ftr_sort_buckets(const CellEntry<D>* in, const long long* n_in, const int* slot_of,
+                                   const long long* boff, CellEntry<D>* out)
 {
+    const long long n = *n_in;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
         const CellEntry<D> me = in[k];
         const int s = slot_of[me.idx];
@@ -1519,21 +1609,36 @@ __global__ void k_ftr_graph_next(FtrLoopArgs<D>* a, cudaGraphConditionalHandle h
 }
 
 #if MCE_COMMON_UNIT
-__global__ void k_group_count(const int* status, const int* owner, long long nR, int* gcnt)
+// Per record: a member counts into its group (gcnt), a root is flagged with
+// its table's capacity, and nothing is alive yet.
+__global__ void k_group_count(const int* status, const int* owner, const int* m, long long nR, int D, int* gcnt,
+                              int* is_root, int* cap, int* alive)
 {
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < nR; j += (long long)gridDim.x * blockDim.x)
-        if (status[j] == 2) atomicAdd(&gcnt[owner[j]], 1);
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t0 == 0) alive[nR] = 0;
+    for (long long j = t0; j < nR; j += (long long)gridDim.x * blockDim.x) {
+        const int st = status[j];
+        if (st == 2) atomicAdd(&gcnt[owner[j]], 1);
+        is_root[j] = st == 1 ? 1 : 0;
+        cap[j] = st == 1 ? half_cells_cap(m[j], D) : 0;
+        alive[j] = 0;
+    }
 }
 
+// Members into their groups' slots (any order), roots into the root list.
 __global__ void k_group_fill(const int* status, const int* owner, long long nR, const long long* goff, int* gfill,
-                             int* members)
+                             int* members, const long long* rscan, int* roots)
 {
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < nR; j += (long long)gridDim.x * blockDim.x)
-        if (status[j] == 2) {
+    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < nR; j += (long long)gridDim.x * blockDim.x) {
+        const int st = status[j];
+        if (st == 2) {
             const int r = owner[j];
             const int k = atomicAdd(&gfill[r], 1);
             members[goff[r] + k] = (int)j;
+        } else if (st == 1) {
+            roots[rscan[j]] = (int)j;
         }
+    }
 }
 
 // Member lists in ascending index order (the forward flag array's order,
@@ -1555,21 +1660,6 @@ __global__ void k_group_sort(const int* gcnt, const long long* goff, long long n
             o[rank] = v;
         }
     }
-}
-
-__global__ void k_roots_flags(const int* status, const int* m, long long nR, int D, int* is_root, int* cap)
-{
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < nR; j += (long long)gridDim.x * blockDim.x) {
-        const bool r = status[j] == 1;
-        is_root[j] = r ? 1 : 0;
-        cap[j] = r ? half_cells_cap(m[j], D) : 0;
-    }
-}
-
-__global__ void k_roots_list(const int* is_root, const long long* rscan, long long nR, int* list)
-{
-    for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < nR; j += (long long)gridDim.x * blockDim.x)
-        if (is_root[j]) list[rscan[j]] = (int)j;
 }
 
 #endif  // MCE_COMMON_UNIT
@@ -1781,7 +1871,7 @@ template <int D>
 __global__ void k_gtable_prep(GCtx c, const int* roots_list, long long nroots, const int* gcnt, const long long* goff,
                               const int* members, const long long* toff, Tables Tnew, int* gnr, int* gitems,
                               int* gcells, int* minfo, double* rps2, double* mps2, int* rflag, int* mflag,
-                              int* need, int* over)
+                              int* pr_mcnt, int* pr_cells, int* pr_items, int* need, int* over)
 {
     extern __shared__ unsigned smem_g[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwb = blockDim.x >> 5;
@@ -1824,6 +1914,7 @@ __global__ void k_gtable_prep(GCtx c, const int* roots_list, long long nroots, c
             gcells[ri] = flat ? nR : 0;
             rps2[ri] = R.ps2[r];
             rflag[ri] = 0;
+            pr_mcnt[ri] = pr_cells[ri] = pr_items[ri] = 0;
         }
         const long long mb = goff[r];
         for (int j = lane; j < nmem; j += 32) {
@@ -2576,11 +2667,12 @@ void Kernels<D>::moments(const double* contrib, long long pitch, const long long
 }
 
 template <int D>
-void Kernels<D>::ftr_cells(TermRecs R, long long nR, long long hmask, int* slot_of, int* bcount, const LaunchCfg& c)
+void Kernels<D>::ftr_cells(TermRecs R, long long nR, long long hmask, int* slot_of, int* bcount, const FtrInit& z,
+                           const LaunchCfg& c)
 {
     if (nR == 0) return;
     ++g_launches;
-    k_ftr_count_cells<D><<<grid_for(nR, 256, c.num_sms), 256, 0, c.stream>>>(R, nR, hmask, slot_of, bcount);
+    k_ftr_count_cells<D><<<grid_for(nR, 256, c.num_sms), 256, 0, c.stream>>>(R, nR, hmask, slot_of, bcount, z);
 }
 
 template <int D>
@@ -2600,12 +2692,12 @@ size_t Kernels<D>::cell_entry_bytes()
 }
 
 template <int D>
-void Kernels<D>::ftr_sort(const void* in, long long n, const int* slot_of, const long long* boff, void* out,
-                          const LaunchCfg& c)
+void Kernels<D>::ftr_sort(const void* in, long long n_bound, const long long* n, const int* slot_of,
+                          const long long* boff, void* out, const LaunchCfg& c)
 {
-    if (n == 0) return;
+    if (n_bound == 0) return;
     ++g_launches;
-    k_ftr_sort_buckets<D><<<grid_for(n, 256, c.num_sms), 256, 0, c.stream>>>(
+    k_ftr_sort_buckets<D><<<grid_for(n_bound, 256, c.num_sms), 256, 0, c.stream>>>(
         static_cast<const CellEntry<D>*>(in), n, slot_of, boff, static_cast<CellEntry<D>*>(out));
 }
 
@@ -2853,7 +2945,7 @@ void Kernels<D>::gtable_prep(TermRecs R, const int* roots_list, long long nroots
     ++g_launches;
     k_gtable_prep<D><<<grid, warps * 32, sm, c.stream>>>(
         ctx, roots_list, nroots, gcnt, goff, members, toff, Tnew, f.gnr, gitems, gcells, f.minfo, f.rps2, f.mps2,
-        f.rflag, f.mflag, need, over);
+        f.rflag, f.mflag, f.pr_mcnt, f.pr_cells, f.pr_items, need, over);
 }
 
 template <int D>
@@ -3774,18 +3866,21 @@ void rel2d_moments(const double* mrows, long long n, long long chunk, double* pa
 #endif  // MCE_COMMON_UNIT
 
 #if MCE_COMMON_UNIT
-void group_count(const int* status, const int* owner, long long nR, int* gcnt, const LaunchCfg& c)
+void group_count(const int* status, const int* owner, const int* m, long long nR, int D, int* gcnt, int* is_root,
+                 int* cap, int* alive, const LaunchCfg& c)
 {
     if (nR == 0) return;
     ++g_launches;
-    k_group_count<<<grid_for(nR, 256, c.num_sms), 256, 0, c.stream>>>(status, owner, nR, gcnt);
+    k_group_count<<<grid_for(nR, 256, c.num_sms), 256, 0, c.stream>>>(status, owner, m, nR, D, gcnt, is_root, cap,
+                                                                      alive);
 }
 void group_fill(const int* status, const int* owner, long long nR, const long long* goff, int* gfill, int* members,
-                const LaunchCfg& c)
+                const long long* rscan, int* roots, const LaunchCfg& c)
 {
     if (nR == 0) return;
     ++g_launches;
-    k_group_fill<<<grid_for(nR, 256, c.num_sms), 256, 0, c.stream>>>(status, owner, nR, goff, gfill, members);
+    k_group_fill<<<grid_for(nR, 256, c.num_sms), 256, 0, c.stream>>>(status, owner, nR, goff, gfill, members, rscan,
+                                                                     roots);
 }
 void group_sort(const int* gcnt, const long long* goff, long long nR, const int* members_in, int* members_out,
                 const LaunchCfg& c)
@@ -3793,18 +3888,6 @@ void group_sort(const int* gcnt, const long long* goff, long long nR, const int*
     if (nR == 0) return;
     ++g_launches;
     k_group_sort<<<grid_for(nR, 8, c.num_sms), 256, 0, c.stream>>>(gcnt, goff, nR, members_in, members_out);
-}
-void roots_flags(const int* status, const int* m, long long nR, int D, int* is_root, int* cap, const LaunchCfg& c)
-{
-    if (nR == 0) return;
-    ++g_launches;
-    k_roots_flags<<<grid_for(nR, 256, c.num_sms), 256, 0, c.stream>>>(status, m, nR, D, is_root, cap);
-}
-void roots_list(const int* is_root, const long long* rscan, long long nR, int* list, const LaunchCfg& c)
-{
-    if (nR == 0) return;
-    ++g_launches;
-    k_roots_list<<<grid_for(nR, 256, c.num_sms), 256, 0, c.stream>>>(is_root, rscan, nR, list);
 }
 long long partition_tiles_cap(long long nR, int E) { return nR / kPartTile + E + 1; }
 

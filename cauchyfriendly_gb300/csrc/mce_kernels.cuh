@@ -102,12 +102,21 @@ int nd_pdf_eval(const NdInput& in, const double* x_host, int npts, double* out_h
 
 // Scratch for the device-wide scans.
 struct ScanScratch {
-    long long* block_sums;  // capacity >= ceil(n / 2048) + 1 at every level
+    long long* block_sums;  // capacity >= ceil(n / 2048) + 1 at every level, for every array of a scan_many
     long long cap;
 };
 
 // out[i] = sum_{k<i} in[k] for i in [0, n]; out[n] holds the total.
 void scan_int_to_ll(const int* in, long long* out, long long n, ScanScratch& s, const LaunchCfg& c);
+// The same for up to kScanJobs arrays of n values at once; total (or null)
+// also receives the sum (page-locked host memory, say).
+struct ScanJob {
+    const int* in;
+    long long* out;
+    long long* total;
+};
+constexpr int kScanJobs = 4;
+void scan_many(const ScanJob* jobs, int njobs, long long n, ScanScratch& s, const LaunchCfg& c);
 
 // Relative-then-transformed 2-D system of two estimators
 // (cauchy_prediction.hpp:306-971).  Pairs are numbered in the reference's
@@ -142,6 +151,16 @@ struct Rel2DArgs {
 // first wall's sine and cosine, gamma1 re, gamma2 re, g (re, im); the last wall
 __host__ __device__ inline int marg2d_stride(int C) { return 6 * C + 5; }
 __host__ __device__ inline int rel2d_stride(int CC) { return marg2d_stride(CC); }
+
+// What the term reduction and the groups after it need zeroed, per record
+// (status -1 for records of no estimator) and the rounds' counts cnt[ncnt].
+struct FtrInit {
+    int* status;
+    int* gcnt;
+    int* gfill;
+    int* cnt;
+    int ncnt;
+};
 
 // bucket positions kept per record between term-reduction rounds
 constexpr int kFtrResume = 8;
@@ -180,12 +199,14 @@ struct Kernels {
                         long long rows_hi, double* tot, cd* est_raw, double* gscale, const LaunchCfg& c);
     // Fast term reduction (term_reduction.hpp:159-276) over the post-MU records:
     // grid cells of b, counting-sorted buckets, near predecessors.
-    static void ftr_cells(TermRecs R, long long nR, long long hmask, int* slot_of, int* bcount, const LaunchCfg& c);
+    static void ftr_cells(TermRecs R, long long nR, long long hmask, int* slot_of, int* bcount, const FtrInit& z,
+                          const LaunchCfg& c);
     static void ftr_scatter(TermRecs R, long long nR, const int* slot_of, const long long* boff, int* bfill,
                             void* ent, const LaunchCfg& c);
     static size_t cell_entry_bytes();
-    static void ftr_sort(const void* in, long long n, const int* slot_of, const long long* boff, void* out,
-                         const LaunchCfg& c);
+    // n: the number of entries, read on the device; n_bound bounds it
+    static void ftr_sort(const void* in, long long n_bound, const long long* n, const int* slot_of,
+                         const long long* boff, void* out, const LaunchCfg& c);
     // One resolution round: over every record (wl_in null) or over the
     // worklist of records still waiting, whose length the kernel reads from
     // n_in (device memory, written by the previous round; n_bound, known on
@@ -259,7 +280,8 @@ struct Kernels {
 };
 
 // Shape-agnostic kernels.
-void group_count(const int* status, const int* owner, long long nR, int* gcnt, const LaunchCfg& c);
+void group_count(const int* status, const int* owner, const int* m, long long nR, int D, int* gcnt, int* is_root,
+                 int* cap, int* alive, const LaunchCfg& c);
 // The pdf grids' split of n terms over npts points: nch chunks of `chunk`
 // terms per point, their sums in part[nch * npts].
 struct PdfChunks {
@@ -285,13 +307,10 @@ void rel2d_compact(const int* keep, const long long* kpos, long long n, long lon
 // relative moments: the 14 columns of mrows summed over the pairs in order
 // (chunks of `chunk` pairs, then the chunk sums), finalised into out[14]
 void rel2d_moments(const double* mrows, long long n, long long chunk, double* part, double* out, const LaunchCfg& c);
-void group_fill(const int* status, const int* owner, long long nR, const long long* goff, int* gfill,
-                int* members, const LaunchCfg& c);
+void group_fill(const int* status, const int* owner, long long nR, const long long* goff, int* gfill, int* members,
+                const long long* rscan, int* roots, const LaunchCfg& c);
 void group_sort(const int* gcnt, const long long* goff, long long nR, const int* members_in, int* members_out,
                 const LaunchCfg& c);
-void roots_flags(const int* status, const int* m, long long nR, int D, int* is_root, int* cap,
-                 const LaunchCfg& c);
-void roots_list(const int* is_root, const long long* rscan, long long nR, int* list, const LaunchCfg& c);
 // Stable partition of the surviving records of each estimator by shape:
 // tiles of records within each estimator (at most partition_tiles_cap(nR, E)
 // of them), per-tile shape counts turned into per-tile prefixes (C, in

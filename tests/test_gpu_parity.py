@@ -375,3 +375,33 @@ def test_seven_state_ltv_window_against_oracle():
     orc.close()
     assert [r["Nt"] for r in want][:5] == [8, 36, 192, 678, 3308]
     G.compare_records(got, want, check_terms=False)
+
+
+@pytest.mark.parametrize("n", [682, 683, 1366])
+def test_scans_at_the_edges_of_their_tiles(n):
+    """Batches of 3n terms after the first update, either side of one and two
+    scan tiles of 2,048: estimators at the start, the middle and the end step
+    as they do alone, bit for bit."""
+    CE, BCE = _gpu()
+    from cauchyfriendly_gb300 import workloads as W
+    prob = W.two_state_lti(seed=2, steps=4)
+    ms = oracle.max_shape_of(prob)
+    rp, bp = oracle.draw_reference_constants(5, 2, ms)
+    rng = np.random.Generator(np.random.PCG64(8))
+    z = prob["msmts"][:, 0] + rng.standard_cauchy((n, 4))
+    tile = lambda a: np.broadcast_to(a, (n,) + a.shape)
+    bat = BCE(tile(prob["A0"]), tile(prob["p0"]), tile(prob["b0"]), [4] * n, 2, 0, 1, 1, tile(rp), tile(bp))
+    pick = [0, 1, n // 2, n - 1]
+    alone = [CE(prob["A0"], prob["p0"], prob["b0"], 4, 2, 0, 1, 1, root_point=rp, b_pert=bp) for _ in pick]
+    model = (prob["Phi"], prob["Gamma"], prob["beta"], prob["H"][0], prob["gamma"][0])
+    for k in range(4):
+        bat.step(z[:, k], model[0], model[1], model[2], tile(model[3]), np.full(n, model[4]), shared_model=True)
+        for e, a in zip(pick, alone):
+            a.step(z[e, k], *model)
+            assert bat.num_terms(e) == a.num_terms()
+            mb, ma = bat.moments(e), a.moments()
+            for key in ("raw_fz", "raw_mean", "raw_cov"):
+                assert G.bitwise_equal(np.atleast_1d(mb[key]), np.atleast_1d(ma[key])), (k, e, key)
+    for a in alone:
+        a.close()
+    bat.close()
