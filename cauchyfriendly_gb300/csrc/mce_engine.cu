@@ -532,6 +532,10 @@ public:
     std::vector<int> h_order;       // moment-chain launch order
     DevBuf<int> ftr_cnt;            // worklist lengths of the resolution rounds
     static constexpr int kFtrFirstBatch = 4, kFtrBatch = 2, kFtrCntSlots = 8, kFtrMaxRounds = 100000;
+    // Steps of this many records or more carry the list of records with long
+    // buckets, whose launch (3 us a round when it is empty) a smaller step is
+    // better without.
+    static constexpr long long kLongLists = 1LL << 14;
     // How the resolution rounds after the first run: 0 queued in batches, the
     // host reading the worklist length once per batch; 1 one persistent
     // cooperative launch; 2 a device-side loop in a CUDA graph.  Chosen with
@@ -673,7 +677,7 @@ public:
     bool have_post = false;
     DevBuf<int> pr_root, pr_mb, pr_mcnt, pr_cells, pr_items;
     DevBuf<long long> pr_moff, pr_ioff, pr_coff;
-    DevBuf<int> ftr_wl[2], ftr_resume;
+    DevBuf<int> ftr_wl[2], ftr_long, ftr_resume;
     DevBuf<int> g_nr, g_items, g_cells, g_rflag, g_minfo, g_mflag, nvert, vsv;
     DevBuf<long long> g_ioff, g_coff, voff;
     DevBuf<double> g_rps2, g_mps2;
@@ -955,7 +959,7 @@ public:
         rel(Rb.cmap), rel(Rb.csmap);
         rel(Bcap), rel(Bkeys), rel(kall_scan), rel(nvert), rel(voff), rel(vsv), rel(fam_mom), rel(mu_rows);
         rel(mu_ints), rel(bcount), rel(boff), rel(slot_of), rel(cell_ent), rel(cell_ent2), rel(status);
-        rel(owner), rel(ftr_wl[0]), rel(ftr_wl[1]), rel(ftr_resume), rel(gcnt), rel(gfill), rel(goff), rel(members);
+        rel(owner), rel(ftr_wl[0]), rel(ftr_wl[1]), rel(ftr_long), rel(ftr_resume), rel(gcnt), rel(gfill), rel(goff), rel(members);
         rel(members_tmp), rel(is_root), rel(cap), rel(rscan), rel(toff), rel(roots_list), rel(alive), rel(src);
         rel(tcnt), rel(g_nr), rel(g_items), rel(g_cells), rel(g_ioff), rel(g_coff), rel(g_rps2), rel(g_rflag);
         rel(g_minfo), rel(g_mps2), rel(g_mflag), rel(pr_root), rel(pr_mb), rel(pr_mcnt), rel(pr_cells);
@@ -1443,12 +1447,15 @@ public:
         if ((s = owner.ensure(nR + 1))) return s;
         if ((s = gcnt.ensure(nR + 1))) return s;
         if ((s = gfill.ensure(nR + 1))) return s;
-        if ((s = ftr_cnt.ensure(kFtrCntSlots))) return s;
+        // the rounds' worklist counts and their long-list counts
+        if ((s = ftr_cnt.ensure(2 * kFtrCntSlots))) return s;
+        const bool long_lists = nR >= kLongLists;
+        if (long_lists && (s = ftr_long.ensure(nR + 1))) return s;
         if ((s = ensure_scan_scratch(std::max(nR, H) + 1))) return s;
         MCE_CUDA(cudaMemsetAsync(bcount.ptr, 0, sizeof(int) * 2 * H, lc.stream));
         pbeg(KID_FTR);
         Kernels<D>::ftr_cells(R, nR, H - 1, slot_of.ptr, bcount.ptr,
-                              FtrInit{status.ptr, gcnt.ptr, gfill.ptr, ftr_cnt.ptr, kFtrCntSlots}, lc);
+                              FtrInit{status.ptr, gcnt.ptr, gfill.ptr, ftr_cnt.ptr, 2 * kFtrCntSlots}, lc);
         pend();
         pbeg(KID_SCAN);
         scan_int_to_ll(bcount.ptr, boff.ptr, H, ss, lc);
@@ -1474,7 +1481,8 @@ public:
         // round trip).  The no-allocation step runs the batched rounds.
         pbeg(KID_FTR);
         Kernels<D>::ftr_resolve(R, nR, cell_ent2.ptr, boff.ptr, H - 1, MC, status.ptr, owner.ptr, nullptr, nullptr,
-                                nR, ftr_wl[0].ptr, ftr_cnt.ptr, ftr_resume.ptr, lc);
+                                nR, ftr_wl[0].ptr, ftr_cnt.ptr, ftr_resume.ptr, long_lists ? ftr_long.ptr : nullptr,
+                                ftr_cnt.ptr + kFtrCntSlots, lc);
         const int fmode = ftr_rounds_mode();
         int pst = MCE_ERR_ARG;
         if (fmode == 1)
@@ -1506,11 +1514,16 @@ public:
             pbeg(KID_FTR);
             for (int q = 0; q < K; q++, round++) {
                 int* n_out = ftr_cnt.ptr + round % kFtrCntSlots;
-                if (round >= kFtrCntSlots) MCE_CUDA(cudaMemsetAsync(n_out, 0, sizeof(int), lc.stream));
+                int* n_long = n_out + kFtrCntSlots;
+                if (round >= kFtrCntSlots) {
+                    MCE_CUDA(cudaMemsetAsync(n_out, 0, sizeof(int), lc.stream));
+                    MCE_CUDA(cudaMemsetAsync(n_long, 0, sizeof(int), lc.stream));
+                }
                 Kernels<D>::ftr_resolve(R, nR, cell_ent2.ptr, boff.ptr, H - 1, MC, status.ptr, owner.ptr,
                                         round ? ftr_wl[(round - 1) & 1].ptr : nullptr,
                                         round ? ftr_cnt.ptr + (round - 1) % kFtrCntSlots : nullptr, bound,
-                                        ftr_wl[round & 1].ptr, n_out, ftr_resume.ptr, lc);
+                                        ftr_wl[round & 1].ptr, n_out, ftr_resume.ptr,
+                                        long_lists ? ftr_long.ptr : nullptr, n_long, lc);
             }
             pend();
             MCE_CUDA(cudaMemcpyAsync(unk, ftr_cnt.ptr + (round - 1) % kFtrCntSlots, sizeof(int),

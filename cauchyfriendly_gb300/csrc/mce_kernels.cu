@@ -1399,11 +1399,83 @@ __global__ void k_ftr_sort_buckets(const CellEntry<D>* in, const long long* n_in
 // root, a root, or waits for the next round (wl_out).  A decision is only
 // taken on predecessors that are decided, so the result does not depend on
 // the order the threads run in.
+//
+// A thread looks at kFtrScanMost bucket entries at most in a round of the
+// batched launches; a record that needs more goes to the long list, which
+// k_ftr_resolve_long works off with a warp per record.  Buckets are short but
+// for estimators whose many terms share one b (20,000 entries and more): their
+// threads, a few warps of the whole launch, took 2.2 ms of the 331-estimator
+// batch's last update.  Rounds of a whole pass, scan + long list: 331
+// estimators 4.9 ms without the list, 2.7 with 96 entries, 1.9 with 32; 4,096
+// estimators 18.0, 13.8, 12.5.
+constexpr int kFtrScanMost = 32;
+
+// The distinct buckets around a record's b, in a fixed order: f(q, s) for the
+// q-th bucket s.
+template <int D, typename F>
+__device__ __forceinline__ void ftr_buckets(const TermRecs& R, long long j, int e, int m, long long hmask, F f)
+{
+    long long lo[D], nc[D];
+    int nprobe = 1;
+    for (int a = 0; a < D; a++) {
+        const double b = R.b[j * D + a];
+        lo[a] = cell_of(b - kProbeHalfWidth);
+        const long long hi = cell_of(b + kProbeHalfWidth);
+        nc[a] = hi - lo[a] + 1;
+        if (nc[a] < 1) nc[a] = 1;
+        if (nc[a] > 2) nc[a] = 2;
+        nprobe *= (int)nc[a];
+    }
+    long long seen[1 << (D < 5 ? D : 5)];
+    int nseen = 0;
+    for (int pr = 0; pr < nprobe; pr++) {
+        long long c[D];
+        int rem = pr;
+        for (int a = 0; a < D; a++) {
+            c[a] = lo[a] + (rem % nc[a]);
+            rem /= (int)nc[a];
+        }
+        const long long s = cell_slot<D>(e, m, c, hmask);
+        bool dup = false;
+        for (int q = 0; q < nseen; q++) dup |= seen[q] == s;
+        if (dup) continue;
+        const int q = nseen;
+        if (nseen < (1 << (D < 5 ? D : 5))) seen[nseen++] = s;
+        f(q, s);
+    }
+}
+
+// Whether entry ce is a near predecessor of record j (of keys kj).
+template <int D>
+__device__ __forceinline__ bool ftr_near(const TermRecs& R, const CellEntry<D>& ce, int em, const long long* kj,
+                                         long long j, int m, int MC)
+{
+    if (ce.est_m != em) return false;
+    for (int a = 0; a < D; a++)
+        if (!(ce.lo[a] < kj[a] && kj[a] <= ce.hi[a])) return false;
+    return ftr_near_pm<D>(R, ce.idx, j, m, MC);
+}
+
+// The record's fate from the smallest near root (best) and the smallest
+// undecided near predecessor (minu); true when it must wait.
+__device__ __forceinline__ bool ftr_decide(long long j, int best, int minu, int* status, int* owner)
+{
+    if (best < minu) {
+        owner[j] = best;
+        ((volatile int*)status)[j] = 2;
+    } else if (minu == INT_MAX) {
+        owner[j] = (int)j;
+        ((volatile int*)status)[j] = 1;
+    } else
+        return true;
+    return false;
+}
+
 template <int D>
 __device__ __forceinline__ void ftr_round(const TermRecs& R, long long nR, const CellEntry<D>* ent,
                                           const long long* boff, long long hmask, int MC, int* status, int* owner,
                                           const int* wl_in, const int* n_in, int* wl_out, int* n_out, int* resume,
-                                          long long tid, long long nth)
+                                          long long tid, long long nth, int* wl_long, int* n_long)
 {
     const long long n = wl_in ? (long long)*(volatile const int*)n_in : nR;
     for (long long w = tid; w < n; w += nth) {
@@ -1414,45 +1486,17 @@ __device__ __forceinline__ void ftr_round(const TermRecs& R, long long nR, const
         const int e = R.est[j];
         const int m = R.m[j];
         const int em = (e << 5) | m;
-        double bj[D];
-        long long kj[D], lo[D], nc[D];
-        int nprobe = 1;
-        for (int a = 0; a < D; a++) {
-            bj[a] = R.b[j * D + a];
-            kj[a] = dkey(bj[a]);
-            lo[a] = cell_of(bj[a] - kProbeHalfWidth);
-            const long long hi = cell_of(bj[a] + kProbeHalfWidth);
-            nc[a] = hi - lo[a] + 1;
-            if (nc[a] < 1) nc[a] = 1;
-            if (nc[a] > 2) nc[a] = 2;
-            nprobe *= (int)nc[a];
-        }
+        long long kj[D];
+        for (int a = 0; a < D; a++) kj[a] = dkey(R.b[j * D + a]);
         int best = INT_MAX, minu = INT_MAX;
-        long long seen[1 << (D < 5 ? D : 5)];
-        int nseen = 0;
-        for (int pr = 0; pr < nprobe; pr++) {
-            long long c[D];
-            int rem = pr;
-            for (int a = 0; a < D; a++) {
-                c[a] = lo[a] + (rem % nc[a]);
-                rem /= (int)nc[a];
-            }
-            const long long s = cell_slot<D>(e, m, c, hmask);
-            bool dup = false;
-            for (int q = 0; q < nseen; q++) dup |= seen[q] == s;
-            if (dup) continue;
-            const int q = nseen;
-            if (nseen < (1 << (D < 5 ? D : 5))) seen[nseen++] = s;
+        int left = wl_long ? kFtrScanMost : INT_MAX;
+        ftr_buckets<D>(R, j, e, m, hmask, [&](int q, long long s) {
             const long long kb = boff[s], ke = boff[s + 1];
             long long k = kb + ((wl_in && q < kFtrResume) ? __ldcg(resume + j * kFtrResume + q) : 0);
-            for (; k < ke; k++) {
+            for (; k < ke && left > 0; k++, left--) {
                 const CellEntry<D>& ce = ent[k];
                 if (ce.idx >= j) break;  // ascending: no predecessors beyond
-                if (ce.est_m != em) continue;
-                bool ok = true;
-                for (int a = 0; a < D && ok; a++)
-                    if (!(ce.lo[a] < kj[a] && kj[a] <= ce.hi[a])) ok = false;
-                if (!ok || !ftr_near_pm<D>(R, ce.idx, j, m, MC)) continue;
+                if (!ftr_near<D>(R, ce, em, kj, j, m, MC)) continue;
                 const int st = ((volatile int*)status)[ce.idx];
                 if (st == 2) continue;  // a member: look further
                 if (st == 1) best = ce.idx < best ? ce.idx : best;
@@ -1460,25 +1504,74 @@ __device__ __forceinline__ void ftr_round(const TermRecs& R, long long nR, const
                 break;  // the first non-member near predecessor of this bucket decides it
             }
             if (q < kFtrResume) resume[j * kFtrResume + q] = (int)(k - kb);
-        }
-        if (best < minu) {
-            owner[j] = best;
-            ((volatile int*)status)[j] = 2;
-        } else if (minu == INT_MAX) {
-            owner[j] = (int)j;
-            ((volatile int*)status)[j] = 1;
-        } else
-            wl_out[atomicAdd(n_out, 1)] = (int)j;
+        });
+        if (left <= 0) wl_long[atomicAdd(n_long, 1)] = (int)j;
+        else if (ftr_decide(j, best, minu, status, owner)) wl_out[atomicAdd(n_out, 1)] = (int)j;
+    }
+}
+
+// The records of the long list, a warp each, 32 entries at a time.
+template <int D>
+__global__ void __launch_bounds__(128) k_ftr_resolve_long(TermRecs R, const CellEntry<D>* ent, const long long* boff,
+                                                          long long hmask, int MC, int* status, int* owner,
+                                                          const int* wl_long, const int* n_long, int* wl_out,
+                                                          int* n_out, int* resume)
+{
+    const int lane = threadIdx.x & 31;
+    const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
+    const int n = *n_long;
+    for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += nw) {
+        const long long j = wl_long[w];
+        const int e = R.est[j];
+        const int m = R.m[j];
+        const int em = (e << 5) | m;
+        long long kj[D];
+        for (int a = 0; a < D; a++) kj[a] = dkey(R.b[j * D + a]);
+        int best = INT_MAX, minu = INT_MAX;
+        ftr_buckets<D>(R, j, e, m, hmask, [&](int q, long long s) {
+            const long long kb = boff[s], ke = boff[s + 1];
+            long long k = kb + (q < kFtrResume ? resume[j * kFtrResume + q] : 0);
+            for (;; k += 32) {
+                bool stop = true, hit = false;
+                int idx = INT_MAX, st = 0;
+                if (k + lane < ke) {
+                    const CellEntry<D>& ce = ent[k + lane];
+                    idx = ce.idx;
+                    if (idx < j) {
+                        stop = false;
+                        if (ftr_near<D>(R, ce, em, kj, j, m, MC)) {
+                            st = ((volatile int*)status)[idx];
+                            hit = st != 2;
+                        }
+                    }
+                }
+                const unsigned at = __ballot_sync(kFull, stop || hit);
+                if (!at) continue;
+                const int f = __ffs(at) - 1;
+                if (__shfl_sync(kFull, hit ? 1 : 0, f)) {
+                    idx = __shfl_sync(kFull, idx, f);
+                    st = __shfl_sync(kFull, st, f);
+                    if (st == 1) best = idx < best ? idx : best;
+                    else minu = idx < minu ? idx : minu;
+                }
+                k += f;
+                break;
+            }
+            __syncwarp();
+            if (q < kFtrResume && lane == 0) resume[j * kFtrResume + q] = (int)(k - kb);
+        });
+        __syncwarp();
+        if (lane == 0 && ftr_decide(j, best, minu, status, owner)) wl_out[atomicAdd(n_out, 1)] = (int)j;
     }
 }
 
 template <int D>
 __global__ void k_ftr_resolve_scan(TermRecs R, long long nR, const CellEntry<D>* ent, const long long* boff,
                                    long long hmask, int MC, int* status, int* owner, const int* wl_in, const int* n_in,
-                                   int* wl_out, int* n_out, int* resume)
+                                   int* wl_out, int* n_out, int* resume, int* wl_long, int* n_long)
 {
     ftr_round<D>(R, nR, ent, boff, hmask, MC, status, owner, wl_in, n_in, wl_out, n_out, resume,
-                 blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+                 blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x, wl_long, n_long);
 }
 
 // Grid-wide barrier of a cooperative launch with a bounded wait: bar[0]
@@ -1540,7 +1633,8 @@ __global__ void __launch_bounds__(128) k_ftr_resolve_all(TermRecs R, long long n
         int* n_out = cnt + r % 3;
         const int* n_in = r ? cnt + (r + 2) % 3 : nullptr;
         if (tid == 0) cnt[(r + 1) % 3] = 0;
-        ftr_round<D>(R, nR, ent, boff, hmask, MC, status, owner, wl_in, n_in, wl_out, n_out, resume, tid, nth);
+        ftr_round<D>(R, nR, ent, boff, hmask, MC, status, owner, wl_in, n_in, wl_out, n_out, resume, tid, nth,
+                     nullptr, nullptr);
         if (!grid_barrier(bar, 1LL << 26)) {
             if (threadIdx.x == 0) atomicOr(err, kErrResolveStalled);
             break;
@@ -1589,7 +1683,7 @@ __global__ void __launch_bounds__(128) k_ftr_graph_round(const FtrLoopArgs<D>* a
     const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long nth = (long long)gridDim.x * blockDim.x;
     ftr_round<D>(R, a->nR, a->ent, a->boff, a->hmask, a->MC, a->status, a->owner, wl_in, a->cnt + (r - 1) % 8, wl_out,
-                 a->cnt + r % 8, a->resume, tid, nth);
+                 a->cnt + r % 8, a->resume, tid, nth, nullptr, nullptr);
 }
 
 template <int D>
@@ -2704,7 +2798,7 @@ void Kernels<D>::ftr_sort(const void* in, long long n_bound, const long long* n,
 template <int D>
 void Kernels<D>::ftr_resolve(TermRecs R, long long nR, const void* ent, const long long* boff, long long hmask,
                              int MC, int* status, int* owner, const int* wl_in, const int* n_in, long long n_bound,
-                             int* wl_out, int* n_out, int* resume, const LaunchCfg& c)
+                             int* wl_out, int* n_out, int* resume, int* wl_long, int* n_long, const LaunchCfg& c)
 {
     const long long n = wl_in ? n_bound : nR;
     if (n == 0) return;
@@ -2713,8 +2807,13 @@ void Kernels<D>::ftr_resolve(TermRecs R, long long nR, const void* ent, const lo
     const TuneLaunch t = tune_begin(TK_FTR_RESOLVE, D, MC, n, 128, mb, c.stream);
     k_ftr_resolve_scan<D><<<tuned_grid(n, t.block, c.num_sms, 16), t.block, 0, c.stream>>>(
         R, nR, static_cast<const CellEntry<D>*>(ent), boff, hmask, MC, status, owner, wl_in, n_in, wl_out, n_out,
-        resume);
+        resume, wl_long, n_long);
     tune_end(t, c.stream);
+    if (!wl_long) return;
+    ++g_launches;
+    k_ftr_resolve_long<D><<<c.num_sms * 4, 128, 0, c.stream>>>(R, static_cast<const CellEntry<D>*>(ent), boff, hmask,
+                                                               MC, status, owner, wl_long, n_long, wl_out, n_out,
+                                                               resume);
 }
 
 template <int D>

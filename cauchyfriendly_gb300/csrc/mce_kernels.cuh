@@ -213,9 +213,11 @@ struct Kernels {
     // the host, bounds it and sizes the grid); the ones that must wait again
     // are appended to wl_out (count n_out); resume holds kFtrResume bucket
     // positions per record.  Rounds thus queue back to back without the host.
+    // wl_long, n_long (or null): a list for the records whose buckets are too
+    // long for a thread, worked off by a second launch of the round.
     static void ftr_resolve(TermRecs R, long long nR, const void* ent, const long long* boff, long long hmask, int MC,
                             int* status, int* owner, const int* wl_in, const int* n_in, long long n_bound,
-                            int* wl_out, int* n_out, int* resume, const LaunchCfg& c);
+                            int* wl_out, int* n_out, int* resume, int* wl_long, int* n_long, const LaunchCfg& c);
     // the resolution rounds from first_round on in one persistent cooperative
     // launch (round r: worklist wl[r & 1], count cnt[r % 3]; the counts
     // zeroed, barrier state bar[2] zeroed); MCE_ERR_CUDA when the cooperative
