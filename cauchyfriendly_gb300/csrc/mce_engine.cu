@@ -2354,8 +2354,8 @@ struct mce_rel2d {
     LaunchCfg lc{};
     int full = 0, CC = 0;
     long long npairs = 0, nkept = 0;
-    DevBuf<double> tt, mrows, mpart, mout, trel, nu, part, xs, ys, zs;
-    DevBuf<int> keep, bad;
+    DevBuf<double> tt, mrows, mpart, mout, trel, nu, part, xs, ys, zs, rowsP, rowsS;
+    DevBuf<int> keep, bad, hdrP, hdrS;
     DevBuf<long long> idxP, idxS, kpos, kidx, scan_tmp;
     DevBuf<Rel2DBlock> blk;
     // device time of the last pair pass, moment sum and grid (CUDA events on the stream)
@@ -2466,6 +2466,16 @@ int rel2d_build(mce_rel2d* r, EngineBase& P, int ep, EngineBase& S, int es, cons
     a.tt = r->tt.ptr;
     a.keep = r->keep.ptr;
     a.mrows = mom ? r->mrows.ptr : nullptr;
+    a.nP = (int)vp.idx.size();
+    a.nS = (int)vs.idx.size();
+    if ((s = r->rowsP.ensure(((size_t)a.nP + 1) * vp.MC * kRelRow))) return s;
+    if ((s = r->rowsS.ensure(((size_t)a.nS + 1) * vs.MC * kRelRow))) return s;
+    if ((s = r->hdrP.ensure(((size_t)a.nP + 1) * kRelHdr))) return s;
+    if ((s = r->hdrS.ensure(((size_t)a.nS + 1) * kRelHdr))) return s;
+    a.rowsP = r->rowsP.ptr;
+    a.rowsS = r->rowsS.ptr;
+    a.hdrP = r->hdrP.ptr;
+    a.hdrS = r->hdrS.ptr;
     MCE_CUDA(cudaEventRecord(r->ev[0], st));
     P.rel2d_pairs(a, st);
     MCE_CUDA(cudaEventRecord(r->ev[1], st));

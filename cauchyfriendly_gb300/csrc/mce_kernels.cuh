@@ -146,7 +146,11 @@ struct Rel2DArgs {
     double* tt;             // npairs x rel2d_stride(CC)
     int* keep;              // npairs: 0 where the term was approximated out
     double* mrows;          // npairs x 14: g, g y_j, -(g y_j y_k) as (re, im)
+    int nP, nS;             // terms of idxP, idxS
+    double *rowsP, *rowsS;  // their rows' shares (n x MC x kRelRow), filled by rel2d_pairs
+    int *hdrP, *hdrS;       // and headers (n x kRelHdr)
 };
+constexpr int kRelRow = 10, kRelHdr = 4;
 // doubles per record of a 2-D term of at most C cells: m, b[2], per cell its
 // first wall's sine and cosine, gamma1 re, gamma2 re, g (re, im); the last wall
 __host__ __device__ inline int marg2d_stride(int C) { return 6 * C + 5; }
