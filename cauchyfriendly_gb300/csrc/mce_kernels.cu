@@ -3824,7 +3824,7 @@ __device__ inline double marg2d_cell(double s1, double c1, double s2, double c2,
     }
     cd cell;
     if (fast) {
-        gamma2 = cmul(gamma2, gamma1);
+        gamma2 = cmul_i(gamma2, gamma1);
         gamma1 = cmul(gamma1, gamma1);
         const cd lo = rdiv(s1, cadd(cscale_i(gamma1, c1), cscale_i(gamma2, s1)));
         const cd hi = rdiv(s2, cadd(cscale_i(gamma1, c2), cscale_i(gamma2, s2)));

@@ -384,22 +384,95 @@ __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const doubl
 
 __device__ inline int nd_remove_bit(int b, int bit) { return ((b >> (bit + 1)) << bit) | (b & ((1 << bit) - 1)); }
 
-// Children of at most lc rows, a thread each: no cells below lc rows (they
-// evaluate to zero and are not carried, cpdf_ndim.hpp:773-776), the
-// 2^lc / 2 trivial cells at lc rows (cell_enumeration.hpp:1129-1136).  The
-// others are flagged for the warp-per-child enumeration.
+// Cells of a child whose parent has at most kNdThreadRows rows, by one thread:
+// the parent's keys (half storage: the top bit clear) are a set of at most 128
+// bits, the child's of 64, in registers.  A warp per child (k_nd_cells) had 22
+// to 29 keys for its 32 lanes and spent its time on bitmaps and barriers: the
+// two-dimensional level of 256 points of a 4-state estimator took 37 ms.
+constexpr int kNdThreadRows = 8;
+
+__device__ inline unsigned long long nd_child_cells(const NdKids& K, long long c, int MC, const long long* ptoff,
+                                                    const int* ptcnt, const int* pkeys)
+{
+    const long long par = K.par[c];
+    const int phc = K.phc[c], z = K.z[c];
+    const int top = 1 << (phc - 1), rev = (1 << phc) - 1, mz = 1 << z;
+    int lhp = K.lhp[c];
+    if (lhp & top) lhp ^= rev;
+    const bool coal = K.hcm[c] != 0;
+    unsigned firsts = 0;  // first row of every coalignment group (cell_enumeration.hpp:1228-1240)
+    if (coal) {
+        const unsigned char* cm = K.cmap + c * MC;
+        const int mpre = K.mpre[c];
+        unsigned seen = 0;
+        for (int j = 0; j < mpre; j++) {
+            const int ci = cm[j];
+            if (ci < 32 && !((seen >> ci) & 1u)) {
+                seen |= 1u << ci;
+                firsts |= 1u << j;
+            }
+        }
+    }
+    const int* pk = pkeys + ptoff[par];
+    const int np = ptcnt[par];
+    unsigned long long p0 = 0, p1 = 0, cells = 0;
+    for (int k = 0; k < np; k++) {
+        const int b = pk[k] ^ lhp;
+        const unsigned long long bit = 1ull << (b & 63);
+        if (b & 64) p1 |= bit;
+        else p0 |= bit;
+    }
+    const bool last = z == phc - 1;
+    for (int k = 0; k < np; k++) {
+        const int b = pk[k] ^ lhp;
+        int bq = b ^ mz;
+        if (last) bq ^= rev;
+        if (!((((bq & 64) ? p1 : p0) >> (bq & 63)) & 1ull)) continue;
+        int key = nd_remove_bit(b, z);
+        if (last) {
+            const int c2 = nd_remove_bit(bq, z);
+            if (c2 < key) key = c2;
+        }
+        if (coal) {
+            int bc = 0, l = 0;
+            for (unsigned f = firsts; f; f &= f - 1, l++)
+                if (key & (int)(f & (0u - f))) bc |= 1 << l;
+            key = bc;
+        }
+        cells |= 1ull << (key & 63);
+    }
+    return cells;
+}
+
+// Children a thread can finish: none below lc rows (they evaluate to zero and
+// are not carried, cpdf_ndim.hpp:773-776), the 2^lc / 2 trivial cells at lc
+// rows (cell_enumeration.hpp:1129-1136), nd_child_cells.  The others are
+// flagged for the warp-per-child enumeration.  keys_out null: counts into
+// ccnt; else the ascending keys from coff[c] on.
 template <int LC>
-__global__ void k_nd_cells_small(NdKids K, long long nk, const long long* coff, int* keys_out, int* big)
+__global__ void k_nd_cells_small(NdKids K, long long nk, int MC, const long long* ptoff, const int* ptcnt,
+                                 const int* pkeys, const long long* coff, int* keys_out, int* big)
 {
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nk;
          c += (long long)gridDim.x * blockDim.x) {
         const int m = K.m[c];
-        if (!keys_out) {
-            big[c] = m > LC ? 1 : 0;
-            if (m <= LC) K.ccnt[c] = m < LC ? 0 : (1 << LC) / 2;
-        } else if (m == LC) {
-            for (int k = 0; k < (1 << LC) / 2; k++) keys_out[coff[c] + k] = k;
+        const bool mine = m <= LC || K.phc[c] <= kNdThreadRows;
+        if (!keys_out) big[c] = mine ? 0 : 1;
+        if (!mine) continue;
+        if (m <= LC) {
+            const int n = m < LC ? 0 : (1 << LC) / 2;
+            if (!keys_out) K.ccnt[c] = n;
+            else
+                for (int k = 0; k < n; k++) keys_out[coff[c] + k] = k;
+            continue;
         }
+        unsigned long long cells = nd_child_cells(K, c, MC, ptoff, ptcnt, pkeys);
+        if (!keys_out) {
+            K.ccnt[c] = __popcll(cells);
+            continue;
+        }
+        int* out = keys_out + coff[c];
+        for (; cells; cells &= cells - 1) *out++ = __ffsll((long long)cells) - 1;
     }
 }
 
@@ -646,8 +719,10 @@ constexpr long long kNdFinalChunk = 1LL << 14;  // terms per block of the final 
 // one-dimensional terms; block b takes chunk b - coff[p] of point p (coff:
 // exclusive scan of the points' chunk counts).  Fixed-order tree sums: the
 // result does not depend on the launch.
-__global__ void k_nd_final_partial(NdTerms T, int MC, const int* keys, const cd* vals, const long long* pstart,
-                                   const long long* coff, int npts, cd* partial)
+// The terms are the last level's children as they were evaluated; keep marks
+// those that count.
+__global__ void k_nd_final_partial(NdTerms T, const int* keep, int MC, const int* keys, const cd* vals,
+                                   const long long* pstart, const long long* coff, int npts, cd* partial)
 {
     __shared__ double sre[kNdFinalThreads], sim[kNdFinalThreads];
     const long long b = blockIdx.x;
@@ -662,11 +737,12 @@ __global__ void k_nd_final_partial(NdTerms T, int MC, const int* keys, const cd*
     const long long e = min(pstart[p + 1], a + kNdFinalChunk);
     cd s = mkcd(0, 0);
     for (long long i = a + threadIdx.x; i < e; i += kNdFinalThreads) {
+        const int nc = T.tcnt[i];
+        if (!keep[i] || nc == 0) continue;
         const bool pos_a = T.A[i * MC] > 0;  // A is [MC][1]: row 0 of term i
         const int lp = pos_a ? 1 : 0, lm = pos_a ? 0 : 1;
         const int* k = keys + T.toff[i];
         const cd* v = vals + T.toff[i];
-        const int nc = T.tcnt[i];
         const cd gp = lookup_num(k, v, nc, lp, 1);
         const cd gm = lookup_num(k, v, nc, lm, 1);
         const double p0 = T.p[i * MC], b0 = T.b[i];
@@ -722,8 +798,9 @@ __global__ void k_nd_reorient(const int* m, const double* A, const double* b, lo
 // chunk of one point's terms (ld dimensions, A [MC][ld]): each term's g value
 // at the sign vector of A nu (bit k set where row k . nu < 0).  Chunks as in
 // k_nd_final_partial.
-__global__ void k_nd_final_marg_partial(NdTerms T, int MC, int ld, const double* nu, const int* keys, const cd* vals,
-                                        const long long* pstart, const long long* coff, int npts, cd* partial)
+__global__ void k_nd_final_marg_partial(NdTerms T, const int* keep, int MC, int ld, const double* nu, const int* keys,
+                                        const cd* vals, const long long* pstart, const long long* coff, int npts,
+                                        cd* partial)
 {
     __shared__ double sre[kNdFinalThreads], sim[kNdFinalThreads];
     const long long b = blockIdx.x;
@@ -738,6 +815,7 @@ __global__ void k_nd_final_marg_partial(NdTerms T, int MC, int ld, const double*
     const long long e = min(pstart[p + 1], a + kNdFinalChunk);
     cd s = mkcd(0, 0);
     for (long long i = a + threadIdx.x; i < e; i += kNdFinalThreads) {
+        if (!keep[i] || T.tcnt[i] == 0) continue;
         const int m = T.m[i];
         const double* Ai = T.A + i * MC * ld;
         int enc = 0;
@@ -810,7 +888,7 @@ namespace {
 
 template <int LD>
 int nd_level(NdWork& w, NdTerms P, const int* pkeys, const cd* pvals, long long n, long long npairs, const double* x,
-             int D, int MC, int MB, NdTermBufs& next, int kb, long long* n_next, const LaunchCfg& lc)
+             int D, int MC, int MB, NdTermBufs* next, int kb, long long* n_next, NdTerms* out, const LaunchCfg& lc)
 {
     constexpr int LC = LD - 1;
     int s;
@@ -846,10 +924,10 @@ int nd_level(NdWork& w, NdTerms P, const int* pkeys, const cd* pvals, long long 
     if ((s = w.big.ensure(nk + 1))) return s;
     if ((s = w.blist.ensure(nk + 1))) return s;
     if ((s = w.ensure_scan(nk + 1))) return s;
-    // the children of at most lc rows a thread each; the others listed for
-    // the warp-per-child enumeration (in 1-D nearly every child coaligns to
-    // one row)
-    k_nd_cells_small<LC><<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(K, nk, nullptr, nullptr, w.big.ptr);
+    // the children a thread can finish; the others listed for the
+    // warp-per-child enumeration (in 1-D nearly every child coaligns to one row)
+    k_nd_cells_small<LC><<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(K, nk, MC, P.toff, P.tcnt, pkeys, nullptr,
+                                                                            nullptr, w.big.ptr);
     scan_int_to_ll(w.big.ptr, w.kscan.ptr, nk, w.ss, lc);
     k_nd_list<<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(w.big.ptr, w.kscan.ptr, nk, w.blist.ptr);
     const long long* nlist = w.kscan.ptr + nk;
@@ -862,13 +940,20 @@ int nd_level(NdWork& w, NdTerms P, const int* pkeys, const cd* pvals, long long 
     w.launches += 3;
     if ((s = w.keys[kb].ensure(ncell + 1))) return s;
     if ((s = w.vals[kb].ensure(ncell + 1))) return s;
-    k_nd_cells_small<LC><<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(K, nk, w.cellof.ptr, w.keys[kb].ptr,
-                                                                            nullptr);
+    k_nd_cells_small<LC><<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(K, nk, MC, P.toff, P.tcnt, pkeys,
+                                                                            w.cellof.ptr, w.keys[kb].ptr, nullptr);
     k_nd_cells<LC><<<cgrid, warps * 32, sm, lc.stream>>>(P.toff, P.tcnt, pkeys, K, w.blist.ptr, nlist, MC, MB,
                                                          w.cellof.ptr, w.keys[kb].ptr);
     if (ncell > 0)
         k_nd_gvals<LC><<<nd_grid(ncell, thr, lc.num_sms), thr, 0, lc.stream>>>(
             P.toff, P.tcnt, pkeys, pvals, K, nk, MC, w.cellof.ptr, ncell, w.keys[kb].ptr, w.vals[kb].ptr);
+    if (!next) {
+        // the last level: its sums read the children where they are
+        *out = NdTerms{K.pt, K.m, K.A, K.p, K.b, w.cellof.ptr, K.ccnt};
+        *n_next = nk;
+        w.launches += 2;
+        return MCE_OK;
+    }
     // the kept children, compacted in order
     if ((s = w.keep_i.ensure(nk + 1))) return s;
     k_nd_keep_int<<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(K, nk, w.keep_i.ptr);
@@ -877,28 +962,29 @@ int nd_level(NdWork& w, NdTerms P, const int* pkeys, const cd* pvals, long long 
     ND_CUDA(cudaMemcpyAsync(&nn, w.kscan.ptr + nk, sizeof(long long), cudaMemcpyDeviceToHost, lc.stream));
     ND_CUDA(cudaStreamSynchronize(lc.stream));
     w.launches += 5;
-    if ((s = next.ensure(nn, MC, LC))) return s;
+    if ((s = next->ensure(nn, MC, LC))) return s;
     if (nn > 0) {
         k_nd_compact<LC><<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(K, nk, MC, w.kscan.ptr,
-                                                                            w.cellof.ptr, next.view());
+                                                                            w.cellof.ptr, next->view());
         w.launches += 1;
     }
+    *out = next->view();
     *n_next = nn;
     return MCE_OK;
 }
 
 int nd_level_dispatch(int LD, NdWork& w, NdTerms P, const int* pkeys, const cd* pvals, long long n,
-                      long long npairs, const double* x, int D, int MC, int MB, NdTermBufs& next, int kb,
-                      long long* n_next, const LaunchCfg& lc)
+                      long long npairs, const double* x, int D, int MC, int MB, NdTermBufs* next, int kb,
+                      long long* n_next, NdTerms* out, const LaunchCfg& lc)
 {
     switch (LD) {
-    case 2: return nd_level<2>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, lc);
-    case 3: return nd_level<3>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, lc);
-    case 4: return nd_level<4>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, lc);
-    case 5: return nd_level<5>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, lc);
-    case 6: return nd_level<6>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, lc);
-    case 7: return nd_level<7>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, lc);
-    case 8: return nd_level<8>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, lc);
+    case 2: return nd_level<2>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, out, lc);
+    case 3: return nd_level<3>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, out, lc);
+    case 4: return nd_level<4>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, out, lc);
+    case 5: return nd_level<5>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, out, lc);
+    case 6: return nd_level<6>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, out, lc);
+    case 7: return nd_level<7>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, out, lc);
+    case 8: return nd_level<8>(w, P, pkeys, pvals, n, npairs, x, D, MC, MB, next, kb, n_next, out, lc);
     default: return MCE_ERR_ARG;
     }
 }
@@ -989,9 +1075,10 @@ int nd_pdf_chunk(const NdInput& in, const double* x_host, int npts, double* out_
     for (int ld = D; ld > stop && !empty; ld--) {
         const bool first = ld == D;
         long long nn = 0;
-        NdTermBufs& next = w->lev[cur];
+        const bool last = ld - 1 == stop;
+        NdTerms next{};
         s = nd_level_dispatch(ld, *w, P, pkeys, pvals, n, first ? n * npts : n, first ? w->x.ptr : nullptr, D, MC,
-                              in.MB, next, cur, &nn, lc);
+                              in.MB, last ? nullptr : &w->lev[cur], cur, &nn, &next, lc);
         if (s) return s;
         int err = 0;
         ND_CUDA(cudaMemcpyAsync(&err, w->err.ptr, sizeof(int), cudaMemcpyDeviceToHost, lc.stream));
@@ -1001,7 +1088,7 @@ int nd_pdf_chunk(const NdInput& in, const double* x_host, int npts, double* out_
                          "(the reference exits, cauchy_term.hpp:673-687)");
             return MCE_ERR_DEVICE;
         }
-        P = next.view();
+        P = next;
         pkeys = w->keys[cur].ptr;
         pvals = w->vals[cur].ptr;
         n = nn;
@@ -1034,9 +1121,10 @@ int nd_pdf_chunk(const NdInput& in, const double* x_host, int npts, double* out_
                 ND_CUDA(cudaMemcpyAsync(w->nu.ptr, in.nu_bar, sizeof(double) * stop, cudaMemcpyHostToDevice,
                                         lc.stream));
                 k_nd_final_marg_partial<<<(unsigned)nb, kNdFinalThreads, 0, lc.stream>>>(
-                    P, MC, stop, w->nu.ptr, pkeys, pvals, w->pstart.ptr, w->pcoff.ptr, npts, w->partial.ptr);
+                    P, w->kids.keep.ptr, MC, stop, w->nu.ptr, pkeys, pvals, w->pstart.ptr, w->pcoff.ptr, npts, w->partial.ptr);
             } else
-                k_nd_final_partial<<<(unsigned)nb, kNdFinalThreads, 0, lc.stream>>>(P, MC, pkeys, pvals, w->pstart.ptr,
+                k_nd_final_partial<<<(unsigned)nb, kNdFinalThreads, 0, lc.stream>>>(P, w->kids.keep.ptr, MC, pkeys, pvals,
+                                                                                     w->pstart.ptr,
                                                                                      w->pcoff.ptr, npts, w->partial.ptr);
         }
         k_nd_final_combine<<<(npts + 127) / 128, 128, 0, lc.stream>>>(w->partial.ptr, w->pcoff.ptr, npts, in.fz, sc,
