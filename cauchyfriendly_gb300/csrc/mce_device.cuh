@@ -215,7 +215,13 @@ __device__ inline float trunc32(double x)
 template <int D>
 __device__ inline int coalign_gate(const double* r, const double* c)
 {
-    {
+    if (D == 1) {
+        // normalised rows of one entry are 1 or -1 (or not a number)
+        const unsigned a = (unsigned)__double2hiint(r[0]), b = (unsigned)__double2hiint(c[0]);
+        if ((a & 0x7fffffffu) == 0x3ff00000u && (b & 0x7fffffffu) == 0x3ff00000u && __double2loint(r[0]) == 0 &&
+            __double2loint(c[0]) == 0)
+            return a == b ? 1 : -1;
+    } else {
         const float a = trunc32(r[0]), b = trunc32(c[0]);
         if (fabsf(a - b) > 3e-7f && fabsf(a + b) > 3e-7f) return 0;
     }

@@ -114,6 +114,7 @@ struct NdKids {
     double* b;        // [lc]
     double* cval;
     double* dval;
+    double* ps2;          // (sum of p)^2, the term-approximation weight
     unsigned char* cmap;  // [MC]
     signed char* csmap;   // [MC]
     int* ccnt;        // cells
@@ -123,7 +124,7 @@ struct NdKidBufs {
     NdBuf<int> pt, m, mpre, phc, z, lhp, hcm, ccnt, keep;
     NdBuf<long long> par;
     NdBuf<unsigned> horthog;
-    NdBuf<double> A, p, q, b, cval, dval;
+    NdBuf<double> A, p, q, b, cval, dval, ps2;
     NdBuf<unsigned char> cmap;
     NdBuf<signed char> csmap;
     int ensure(long long n, int MC, int lc)
@@ -146,6 +147,7 @@ struct NdKidBufs {
         s |= b.ensure((size_t)(n + 1) * std::max(lc, 1));
         s |= cval.ensure(n + 1);
         s |= dval.ensure(n + 1);
+        s |= ps2.ensure(n + 1);
         s |= cmap.ensure((size_t)(n + 1) * MC);
         s |= csmap.ensure((size_t)(n + 1) * MC);
         return s;
@@ -153,8 +155,8 @@ struct NdKidBufs {
     NdKids view()
     {
         return NdKids{pt.ptr,   par.ptr,  m.ptr,     mpre.ptr, phc.ptr,   z.ptr,     lhp.ptr,  horthog.ptr,
-                      hcm.ptr,  A.ptr,    p.ptr,     q.ptr,    b.ptr,     cval.ptr,  dval.ptr, cmap.ptr,
-                      csmap.ptr, ccnt.ptr, keep.ptr};
+                      hcm.ptr,  A.ptr,    p.ptr,     q.ptr,    b.ptr,     cval.ptr,  dval.ptr, ps2.ptr,
+                      cmap.ptr, csmap.ptr, ccnt.ptr, keep.ptr};
     }
 };
 
@@ -185,7 +187,7 @@ __global__ void k_nd_count(NdTerms P, long long n, long long npairs, int MC, int
         if (m >= LD) {
             const double* A = P.A + t * MC * LD;
             for (int r = 0; r < m; r++)
-                if (fabs(A[r * LD + LD - 1]) > kMuEps) c++;
+                if (abs_gt(A[r * LD + LD - 1], kMuEps)) c++;
         }
         cnt[i] = c;
     }
@@ -201,8 +203,8 @@ __device__ int nd_coalign(double* A, double* p, double* q, unsigned& hor, int m,
 {
     for (int i = 0; i < m; i++) {
         q[i] = p[i];
-        double n1 = 0;
-        for (int j = 0; j < LC; j++) n1 += fabs(A[i * LC + j]);
+        double n1 = fabs(A[i * LC]);
+        for (int j = 1; j < LC; j++) n1 += fabs(A[i * LC + j]);
         p[i] *= n1;
         const DivBy by = div_by(n1);
         for (int j = 0; j < LC; j++) A[i * LC + j] = divide(A[i * LC + j], by);
@@ -314,9 +316,9 @@ __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const doubl
         int lam = 0, tz = 0, k = 0;
         for (int r = 0; r < m; r++) {
             Ald[r] = -A[r * LD + LD - 1];
-            nz[r] = fabs(Ald[r]) > kMuEps;
+            nz[r] = abs_gt(Ald[r], kMuEps);
             if (nz[r]) {
-                if (Ald[r] < 0) lam |= 1 << r;
+                if (neg(Ald[r])) lam |= 1 << r;
                 if (k++ == ord) tz = r;
             }
         }
@@ -363,10 +365,13 @@ __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const doubl
         }
         double* Ao = K.A + c * MC * LC;
         for (int q = 0; q < ns * LC; q++) Ao[q] = Ac[q];
+        double ps = 0;
         for (int q = 0; q < ns; q++) {
             K.p[c * MC + q] = pc[q];
             K.q[c * MC + q] = qc[q];
+            ps += pc[q];
         }
+        K.ps2[c] = ps * ps;
         K.pt[c] = pt;
         K.par[c] = t;
         K.m[c] = ns;
@@ -625,11 +630,8 @@ __global__ void k_nd_gvals(const long long* ptoff, const int* ptcnt, const int* 
         const double* q = K.q + c * MC;
         const int be = keys[x];
         double ygi = 0;
-        int sb[kNdMaxRows];
-        for (int k = 0; k < m; k++) {
-            sb[k] = ((be >> k) & 1) ? -1 : 1;
-            if (!hor || !(hor & (1u << k))) ygi += q[k] * sb[k];
-        }
+        for (int k = 0; k < m; k++)
+            if (!(hor & (1u << k))) ygi += ((be >> k) & 1) ? -q[k] : q[k];  // q_k * s_k, exact
         int lp = 0, lm = 0;
         {
             const bool coal = K.hcm[c] != 0;
@@ -642,8 +644,8 @@ __global__ void k_nd_gvals(const long long* ptoff, const int* ptcnt, const int* 
                     k++;
                     if (k == phc) break;
                 }
-                const int bv = coal ? sb[cm[l]] * cs[l] : sb[l];
-                if (bv < 0) {
+                const int r = coal ? cm[l] : l;
+                if ((((be >> r) & 1) != 0) != (coal && cs[l] < 0)) {
                     lp |= 1 << k;
                     lm |= 1 << k;
                 }
@@ -660,13 +662,8 @@ __global__ void k_nd_gvals(const long long* ptoff, const int* ptcnt, const int* 
         const cd gm = lookup_num(pk, pv, np, lm ^ lhp, phc);
         const double cv = K.cval[c], dv = K.dval[c];
         cd v = csub(cdiv(gp, mkcd(ygi + dv, cv)), cdiv(gm, mkcd(ygi - dv, cv)));
-        v = cscale(v, 1.0);
         vals[x] = v;
-        double ps = 0;
-        const double* p = K.p + c * MC;
-        for (int k = 0; k < m; k++) ps += p[k];
-        ps *= ps;
-        if (above_approx_threshold(ps, v.re, v.im)) K.keep[c] = 1;
+        if (above_approx_threshold(K.ps2[c], v.re, v.im)) K.keep[c] = 1;
     }
 }
 
