@@ -102,7 +102,6 @@ struct NdKids {
     int* pt;
     long long* par;   // parent (index into the parent level)
     int* m;           // rows after coalignment
-    int* mpre;        // rows before (parent rows - 1)
     int* phc;         // parent rows (bits of the parent's keys)
     int* z;           // the integrated hyperplane's index in the parent
     int* lhp;         // enc_lambda_bar
@@ -115,24 +114,24 @@ struct NdKids {
     double* cval;
     double* dval;
     double* ps2;          // (sum of p)^2, the term-approximation weight
-    unsigned char* cmap;  // [MC]
-    signed char* csmap;   // [MC]
+    unsigned long long* cmap;  // four bits a row: the coalignment group it belongs to
+    unsigned* csneg;      // the rows against their group's first
+    unsigned* first;      // the groups' first rows
     int* ccnt;        // cells
     int* keep;        // not approximated out
 };
 struct NdKidBufs {
-    NdBuf<int> pt, m, mpre, phc, z, lhp, hcm, ccnt, keep;
+    NdBuf<int> pt, m, phc, z, lhp, hcm, ccnt, keep;
     NdBuf<long long> par;
     NdBuf<unsigned> horthog;
     NdBuf<double> A, p, q, b, cval, dval, ps2;
-    NdBuf<unsigned char> cmap;
-    NdBuf<signed char> csmap;
+    NdBuf<unsigned long long> cmap;
+    NdBuf<unsigned> csneg, first;
     int ensure(long long n, int MC, int lc)
     {
         int s = MCE_OK;
         s |= pt.ensure(n + 1);
         s |= m.ensure(n + 1);
-        s |= mpre.ensure(n + 1);
         s |= phc.ensure(n + 1);
         s |= z.ensure(n + 1);
         s |= lhp.ensure(n + 1);
@@ -148,15 +147,16 @@ struct NdKidBufs {
         s |= cval.ensure(n + 1);
         s |= dval.ensure(n + 1);
         s |= ps2.ensure(n + 1);
-        s |= cmap.ensure((size_t)(n + 1) * MC);
-        s |= csmap.ensure((size_t)(n + 1) * MC);
+        s |= cmap.ensure(n + 1);
+        s |= csneg.ensure(n + 1);
+        s |= first.ensure(n + 1);
         return s;
     }
     NdKids view()
     {
-        return NdKids{pt.ptr,   par.ptr,  m.ptr,     mpre.ptr, phc.ptr,   z.ptr,     lhp.ptr,  horthog.ptr,
+        return NdKids{pt.ptr,   par.ptr,  m.ptr,     phc.ptr,   z.ptr,     lhp.ptr,  horthog.ptr,
                       hcm.ptr,  A.ptr,    p.ptr,     q.ptr,    b.ptr,     cval.ptr,  dval.ptr, ps2.ptr,
-                      cmap.ptr, csmap.ptr, ccnt.ptr, keep.ptr};
+                      cmap.ptr, csneg.ptr, first.ptr, ccnt.ptr, keep.ptr};
     }
 };
 
@@ -197,9 +197,11 @@ __global__ void k_nd_count(NdTerms P, long long n, long long npairs, int MC, int
 // calling thread: rows normalised (q = p first), coaligned rows merged with
 // their p and q, the coalignment maps recorded.  Returns the new row count,
 // or -1 where the reference exits (two unintegrable rows anti-coaligned).
+// (Maps and flags are bit fields: as byte arrays in memory, written a byte at a
+// time, they were most of the kernel's traffic.)
 template <int LC>
-__device__ int nd_coalign(double* A, double* p, double* q, unsigned& hor, int m, unsigned char* cmap,
-                          signed char* csmap)
+__device__ int nd_coalign(double* A, double* p, double* q, unsigned& hor, int m, unsigned long long& cmap,
+                          unsigned& csneg, unsigned& first)
 {
     for (int i = 0; i < m; i++) {
         q[i] = p[i];
@@ -209,64 +211,50 @@ __device__ int nd_coalign(double* A, double* p, double* q, unsigned& hor, int m,
         const DivBy by = div_by(n1);
         for (int j = 0; j < LC; j++) A[i * LC + j] = divide(A[i * LC + j], by);
     }
-    bool F[kNdMaxRows], hf[kNdMaxRows];
-    for (int j = 0; j < m; j++) {
-        F[j] = true;
-        hf[j] = hor ? ((hor >> j) & 1u) : false;
-        cmap[j] = 255;
-        csmap[j] = 1;
-    }
+    unsigned F = (1u << m) - 1u, hf = hor;
+    unsigned long long cm = 0;
+    unsigned cs = 0;
     int uc = 0;
     for (int j = 0; j < m - 1; j++) {
-        if (!F[j]) continue;
-        cmap[j] = (unsigned char)uc;
+        if (!((F >> j) & 1u)) continue;
+        cm |= (unsigned long long)uc << (4 * j);
         for (int k = j + 1; k < m; k++) {
-            if (!F[k]) continue;
+            if (!((F >> k) & 1u)) continue;
             const int g = coalign_gate<LC>(A + j * LC, A + k * LC);
+            if (g == 0) continue;
+            const bool hj = (hf >> j) & 1u, hk = (hf >> k) & 1u;
             if (g == 1) {
-                if (hor) {
-                    const bool hj = hf[j], hk = hf[k];
-                    if (!hj && !hk) q[j] += q[k];
-                    else if (hj && !hk) {
-                        q[j] = q[k];
-                        hf[j] = false;
-                    } else if (!hj && hk) hf[k] = false;
-                    else {
-                        hf[k] = false;
-                        q[j] += q[k];
-                    }
+                if (hor && hj && !hk) {
+                    q[j] = q[k];
+                    hf &= ~(1u << j);
+                } else if (hor && hk) {
+                    if (hj) q[j] += q[k];
+                    hf &= ~(1u << k);
                 } else
                     q[j] += q[k];
-                F[k] = false;
-                p[j] += p[k];
-                cmap[k] = (unsigned char)uc;
-                csmap[k] = 1;
-            } else if (g == -1) {
-                if (hor) {
-                    const bool hj = hf[j], hk = hf[k];
-                    if (!hj && !hk) q[j] -= q[k];
-                    else if (hj && !hk) {
-                        q[j] = -q[k];
-                        hf[j] = false;
-                    } else if (!hj && hk) hf[k] = false;
-                    else return -1;
+            } else {
+                if (hor && hj && !hk) {
+                    q[j] = -q[k];
+                    hf &= ~(1u << j);
+                } else if (hor && hk) {
+                    if (hj) return -1;
+                    hf &= ~(1u << k);
                 } else
                     q[j] -= q[k];
-                F[k] = false;
-                p[j] += p[k];
-                cmap[k] = (unsigned char)uc;
-                csmap[k] = -1;
+                cs |= 1u << k;
             }
+            F &= ~(1u << k);
+            p[j] += p[k];
+            cm |= (unsigned long long)uc << (4 * k);
         }
         uc++;
     }
-    if (F[m - 1]) cmap[m - 1] = (unsigned char)uc;
-    int ns = 0;
-    for (int i = 0; i < m; i++) ns += F[i] ? 1 : 0;
+    if ((F >> (m - 1)) & 1u) cm |= (unsigned long long)uc << (4 * (m - 1));
+    const int ns = __popc(F);
     if (ns != m) {
         int u = 1;
         for (int j = 1; j < m; j++)
-            if (F[j]) {
+            if ((F >> j) & 1u) {
                 if (u < j) {
                     for (int l = 0; l < LC; l++) A[u * LC + l] = A[j * LC + l];
                     p[u] = p[j];
@@ -278,10 +266,13 @@ __device__ int nd_coalign(double* A, double* p, double* q, unsigned& hor, int m,
             unsigned nh = 0;
             int c = 0;
             for (int j = 0; j < m; j++)
-                if (F[j]) nh |= (hf[j] ? 1u : 0u) << c++;
+                if ((F >> j) & 1u) nh |= ((hf >> j) & 1u) << c++;
             hor = nh;
         }
     }
+    cmap = cm;
+    csneg = cs;
+    first = F;
     return ns;
 }
 
@@ -289,7 +280,9 @@ __device__ int nd_coalign(double* A, double* p, double* q, unsigned& hor, int m,
 // the pair i whose children start at coff[i] <= c, and integrates the
 // (c - coff[i])-th of its parent's rows with a nonzero last component.
 // x: the points [npts][D] on the first level, else null.
-template <int LD>
+// MR: the most rows a child can have here (8 or 15), so that the threads' rows
+// stay in the L1.
+template <int LD, int MR>
 __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const double* x, int D, const long long* coff,
                            long long nk, int MC, NdKids K, int* err)
 {
@@ -311,19 +304,18 @@ __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const doubl
         const double* pp = P.p + t * MC;
         const double* bb = P.b + t * LD;
         // construct_lowered_parent_elements (cpdf_ndim.hpp:392-443)
-        double Ald[kNdMaxRows];
-        bool nz[kNdMaxRows];
+        auto ald = [&](int r) { return -A[r * LD + LD - 1]; };
+        unsigned nz = 0;
         int lam = 0, tz = 0, k = 0;
         for (int r = 0; r < m; r++) {
-            Ald[r] = -A[r * LD + LD - 1];
-            nz[r] = abs_gt(Ald[r], kMuEps);
-            if (nz[r]) {
-                if (neg(Ald[r])) lam |= 1 << r;
-                if (k++ == ord) tz = r;
-            }
+            const double v = ald(r);
+            if (!abs_gt(v, kMuEps)) continue;
+            nz |= 1u << r;
+            if (neg(v)) lam |= 1 << r;
+            if (k++ == ord) tz = r;
         }
         double mu_t[LC > 0 ? LC : 1];
-        const DivBy by_t = div_by(Ald[tz]);
+        const DivBy by_t = div_by(ald(tz));
         for (int j = 0; j < LC; j++) mu_t[j] = divide(A[tz * LD + j], by_t);
         double tb;
         double* bo = K.b + c * LC;
@@ -336,15 +328,15 @@ __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const doubl
             for (int j = 0; j < LC; j++) bo[j] = bb[j] + tb * mu_t[j];
         }
         // construct_lowered_children (cpdf_ndim.hpp:579-636): rows mu_l - mu_t
-        double Ac[kNdMaxRows * (LC > 0 ? LC : 1)], pc[kNdMaxRows], qc[kNdMaxRows];
+        double Ac[MR * (LC > 0 ? LC : 1)], pc[MR], qc[MR];
         int l_ = 0;
         unsigned unint = 0;
         for (int l = 0; l < m; l++) {
             if (l == tz) continue;
-            if (nz[l]) {
-                const DivBy by = div_by(Ald[l]);
+            if ((nz >> l) & 1u) {
+                const DivBy by = div_by(ald(l));
                 for (int j = 0; j < LC; j++) Ac[l_ * LC + j] = divide(A[l * LD + j], by) - mu_t[j];
-                pc[l_] = pp[l] * fabs(Ald[l]);
+                pc[l_] = pp[l] * fabs(ald(l));
             } else {
                 for (int j = 0; j < LC; j++) Ac[l_ * LC + j] = A[l * LD + j];
                 pc[l_] = pp[l];
@@ -353,9 +345,9 @@ __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const doubl
             l_++;
         }
         const int mpre = m - 1;
-        unsigned char* cm = K.cmap + c * MC;
-        signed char* cs = K.csmap + c * MC;
-        const int ns = nd_coalign<LC>(Ac, pc, qc, unint, mpre, cm, cs);
+        unsigned long long cm;
+        unsigned cs, first;
+        const int ns = nd_coalign<LC>(Ac, pc, qc, unint, mpre, cm, cs, first);
         if (ns < 0) {
             atomicOr(err, kErrAntiCoalignedHorthog);
             K.m[c] = 0;
@@ -375,14 +367,16 @@ __global__ void k_nd_lower(NdTerms P, long long n, long long npairs, const doubl
         K.pt[c] = pt;
         K.par[c] = t;
         K.m[c] = ns;
-        K.mpre[c] = mpre;
         K.phc[c] = m;
         K.z[c] = tz;
         K.lhp[c] = lam;
         K.horthog[c] = unint;
         K.hcm[c] = ns < mpre ? 1 : 0;
         K.cval[c] = tb;
-        K.dval[c] = pp[tz] * fabs(Ald[tz]);
+        K.dval[c] = pp[tz] * fabs(ald(tz));
+        K.cmap[c] = cm;
+        K.csneg[c] = cs;
+        K.first[c] = first;
         K.keep[c] = 0;
     }
 }
@@ -405,19 +399,7 @@ __device__ inline unsigned long long nd_child_cells(const NdKids& K, long long c
     int lhp = K.lhp[c];
     if (lhp & top) lhp ^= rev;
     const bool coal = K.hcm[c] != 0;
-    unsigned firsts = 0;  // first row of every coalignment group (cell_enumeration.hpp:1228-1240)
-    if (coal) {
-        const unsigned char* cm = K.cmap + c * MC;
-        const int mpre = K.mpre[c];
-        unsigned seen = 0;
-        for (int j = 0; j < mpre; j++) {
-            const int ci = cm[j];
-            if (ci < 32 && !((seen >> ci) & 1u)) {
-                seen |= 1u << ci;
-                firsts |= 1u << j;
-            }
-        }
-    }
+    const unsigned firsts = K.first[c];  // first row of every coalignment group (cell_enumeration.hpp:1228-1240)
     const int* pk = pkeys + ptoff[par];
     const int np = ptcnt[par];
     unsigned long long p0 = 0, p1 = 0, cells = 0;
@@ -536,17 +518,8 @@ __global__ void k_nd_cells(const long long* ptoff, const int* ptcnt, const int* 
         const bool coal = K.hcm[c] != 0;
         if (coal && lane == 0) {
             // first row of every coalignment group (cell_enumeration.hpp:1228-1240)
-            const unsigned char* cm = K.cmap + c * MC;
-            const int mpre = K.mpre[c];
-            unsigned seen = 0;
             int cnt = 0;
-            for (int j = 0; j < mpre; j++) {
-                const int ci = cm[j];
-                if (ci < 32 && !((seen >> ci) & 1u)) {
-                    seen |= 1u << ci;
-                    bmk[cnt++] = j;
-                }
-            }
+            for (unsigned f = K.first[c]; f; f &= f - 1) bmk[cnt++] = __ffs(f) - 1;
             bmk[31] = cnt;
         }
         __syncwarp();
@@ -635,8 +608,8 @@ __global__ void k_nd_gvals(const long long* ptoff, const int* ptcnt, const int* 
         int lp = 0, lm = 0;
         {
             const bool coal = K.hcm[c] != 0;
-            const unsigned char* cm = K.cmap + c * MC;
-            const signed char* cs = K.csmap + c * MC;
+            const unsigned long long cm = K.cmap[c];
+            const unsigned cs = K.csneg[c];
             int k = 0, l = 0;
             while (k < phc) {
                 if (k == z) {
@@ -644,8 +617,8 @@ __global__ void k_nd_gvals(const long long* ptoff, const int* ptcnt, const int* 
                     k++;
                     if (k == phc) break;
                 }
-                const int r = coal ? cm[l] : l;
-                if ((((be >> r) & 1) != 0) != (coal && cs[l] < 0)) {
+                const int r = coal ? (int)(cm >> (4 * l)) & 15 : l;
+                if ((((be >> r) & 1) != 0) != (coal && ((cs >> l) & 1u))) {
                     lp |= 1 << k;
                     lm |= 1 << k;
                 }
@@ -905,8 +878,13 @@ int nd_level(NdWork& w, NdTerms P, const int* pkeys, const cd* pvals, long long 
     }
     if ((s = w.kids.ensure(nk, MC, LC))) return s;
     NdKids K = w.kids.view();
-    k_nd_lower<LD><<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(P, n, npairs, x, D, w.coff.ptr, nk, MC, K,
-                                                                      w.err.ptr);
+    // (no term has more than MB rows, no child more than MB - 1)
+    if (MB <= 9)
+        k_nd_lower<LD, 8><<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(P, n, npairs, x, D, w.coff.ptr, nk, MC,
+                                                                              K, w.err.ptr);
+    else
+        k_nd_lower<LD, 15><<<nd_grid(nk, thr, lc.num_sms), thr, 0, lc.stream>>>(P, n, npairs, x, D, w.coff.ptr, nk, MC,
+                                                                               K, w.err.ptr);
     // cells: counts, offsets, keys
     const int words = (1 << MB) > 32 ? (1 << MB) / 32 : 1;
     const size_t pw = (size_t)(2 * words + 32) * 4;
