@@ -405,3 +405,29 @@ def test_scans_at_the_edges_of_their_tiles(n):
     for a in alone:
         a.close()
     bat.close()
+
+
+@pytest.mark.parametrize("states,updates", [(3, 12), (5, 7)])
+def test_table_cells_at_the_largest_parents_of_the_shared_memory_path(states, updates):
+    """Groups whose cells come from tables in shared memory: three states up
+    to parents of 14 rows, one above that path's limit of 13, and the large
+    groups of five states with two measurements a step, against the oracle
+    (integer structure exact, moments within 1e-9)."""
+    from cauchyfriendly_gb300 import workloads as W
+    prob = W.three_state_lti(seed=1, steps=14) if states == 3 else W.five_state_ltv_windows(seed=0, steps=8)
+    rp, bp = oracle.draw_reference_constants(7, states, oracle.max_shape_of(prob))
+    gpu = _GpuAdapter(prob, rp, bp)
+    orc = oracle.Oracle(prob, rp, bp)
+    got, want = [], []
+    for i in range(updates):
+        for est, out in ((gpu, got), (orc, want)):
+            err = est.step(i // prob["p"], i % prob["p"])
+            rec = est.moments()
+            rec["err"] = int(err)
+            rec["Nt"] = est.num_terms()
+            rec["tps"] = est.terms_per_shape()
+            out.append(rec)
+    assert gpu.est.device_errors() == 0
+    gpu.close()
+    orc.close()
+    G.compare_records(got, want, check_terms=False)
