@@ -708,7 +708,9 @@ public:
     long long p_l0 = 0;
     DevBuf<double> alg;  // [KID_COUNT][2] bytes, flops
     DevBuf<unsigned> gbits;  // cell bitmaps of terms above kSmemBitmapRows hyperplanes
-    DevBuf<int> g_over;      // g-table preparation: a root above its slot, the largest count
+    // g-table preparation: a root above its slot, the largest count, the groups
+    // of many cells; the next of these to be summed
+    DevBuf<int> g_over;
 
     // profiling brackets on the engine's stream (or on st when given)
     void pbeg(int id, cudaStream_t st = nullptr)
@@ -818,7 +820,7 @@ public:
         int s = MCE_OK;
         // profiling counters, sized here so no later step has to allocate them
         s |= alg.ensure(2 * KID_COUNT);
-        s |= g_over.ensure(2);
+        s |= g_over.ensure(4);
         if (MC > kSmemBitmapRows) {
             // a region per warp for the bitmap kernels (8 warps per SM)
             const long long warps = (long long)lc.num_sms * 8;
@@ -1596,20 +1598,22 @@ public:
                  g_mflag.ptr, nullptr,       pr_root.ptr,   pr_mb.ptr,    pr_mcnt.ptr,  pr_cells.ptr,
                  pr_items.ptr, pr_moff.ptr,  pr_ioff.ptr,   pr_coff.ptr,  nullptr};
         Tables Tnv{Tn.keys.ptr, Tn.vals.ptr};
+        long long nbig = 0;
         for (int attempt = 0;; attempt++) {
-            MCE_CUDA(cudaMemsetAsync(g_over.ptr, 0, 2 * sizeof(int), lc.stream));
+            MCE_CUDA(cudaMemsetAsync(g_over.ptr, 0, 4 * sizeof(int), lc.stream));
             pbeg(KID_GTABLE);
             Kernels<D>::gtable_prep(R, roots_list.ptr, nroots, gcnt.ptr, goff.ptr, members.ptr, PV, Told, Bkeys.ptr,
                                     toff.ptr, Tnv, gf, g_items.ptr, g_cells.ptr, MC, cap.ptr, g_over.ptr, lc);
             const ScanJob item_jobs[2] = {{g_items.ptr, g_ioff.ptr, tot + 6}, {g_cells.ptr, g_coff.ptr, tot + 7}};
             scan_many(item_jobs, 2, nroots, ss, lc);
             pend();
-            int* const ov = h_ints.data() + 2;
-            ov[0] = ov[1] = 0;
+            int* const ov = h_ints.data() + 5;
+            ov[0] = ov[1] = ov[2] = 0;
             if (nroots > 0) {
-                MCE_CUDA(cudaMemcpyAsync(ov, g_over.ptr, 2 * sizeof(int), cudaMemcpyDeviceToHost, lc.stream));
+                MCE_CUDA(cudaMemcpyAsync(ov, g_over.ptr, 3 * sizeof(int), cudaMemcpyDeviceToHost, lc.stream));
                 MCE_CUDA(cudaStreamSynchronize(lc.stream));
             }
+            nbig = ov[2];
             if (!ov[0]) break;
             if (attempt > 0) {
                 device_errors |= kErrRootCellsOverflow;
@@ -1656,7 +1660,8 @@ public:
         Kernels<D>::gtable_combine(R, roots_list.ptr, nroots, g_coff.ptr, ncells, gcnt.ptr, goff.ptr, members.ptr, PV,
                                    Told, Bkeys.ptr, toff.ptr, Tnv, tcnt.ptr, alive.ptr, src.ptr, gf, MC, lc);
         Kernels<D>::gtable(R, roots_list.ptr, nroots, gcnt.ptr, goff.ptr, members.ptr, PV, Told, Bkeys.ptr, gscale.ptr,
-                           toff.ptr, Tnv, tcnt.ptr, alive.ptr, src.ptr, gscr, capR, gf, MC, err, lc, gscr_warps);
+                           toff.ptr, Tnv, tcnt.ptr, alive.ptr, src.ptr, gscr, capR, gf, MC, err, nbig, g_over.ptr + 3, lc,
+                           gscr_warps);
         // members left after promotions: the promoted-root flat pass
         const ScanJob prom_jobs[3] = {{pr_mcnt.ptr, pr_moff.ptr, tot + 8},
                                       {pr_items.ptr, pr_ioff.ptr, tot + 9},

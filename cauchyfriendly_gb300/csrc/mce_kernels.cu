@@ -1826,7 +1826,7 @@ __device__ inline cd g_cell(const GCtx& c, long long s, int key, double gscale)
     return cscale(v, gscale);
 }
 
-// g_cell for many cells of one record, by a warp: what depends on the record
+// g_cell for many cells of one record, by a team of W warps: what depends on the record
 // alone is laid out in shared memory first, so that a cell needs no loop over
 // its parent's rows and no binary search.
 //   bits, pref  the parent table's keys (half storage: 2^(phc-1) bits) and the
@@ -1835,28 +1835,46 @@ __device__ inline cd g_cell(const GCtx& c, long long s, int key, double gscale)
 //               lambda keys are a few XORs
 //   T           the partial sums of the first kFastLow rows for all their sign
 //               patterns: a cell's sum goes on from there, in the same order
-// For parents of at most kFastRows rows (the others: g_cell).  Large groups
-// spend their time here: the 5-state sliding windows' k_gtable 117 -> 101 ms.
+// For the large groups, which spend their time here (the 5-state sliding
+// windows' k_gtable 117 -> 101 ms), and parents of at most kFastRows rows; the
+// others use g_cell: in groups of at most kFlatMaxCells cells the set-up costs
+// more than it saves (4,096 3-state estimators: 5.4 ms without, 7.7 ms with).
 constexpr int kFastRows = 13, kFastLow = 7;
 struct GFastSmem {
     double T[1 << kFastLow];
     unsigned bits[(1 << (kFastRows - 1)) / 32];
-    int col[kSmemBitmapRows];
+    int col[kSmemBitmapRows], c0;
     unsigned short pref[(1 << (kFastRows - 1)) / 32];
 };
 
-template <int D>
+// A team of W warps (one group of k_gtable): its barrier and reductions.
+template <int W>
+__device__ inline void team_sync()
+{
+    if (W == 1) __syncwarp();
+    else __syncthreads();
+}
+template <int W>
+__device__ inline bool team_all(bool x)
+{
+    if (W > 1) return __syncthreads_and(x);
+    __syncwarp();
+    return __all_sync(kFull, x);
+}
+
+template <int D, int W>
 struct GFast {
+    static constexpr int kTeam = 32 * W;
     GFastSmem* S;
     bool on, child;
-    int m, phc, low, c0, zbit, lhp;
+    int m, phc, low, zbit, lhp;
     unsigned hof;
     const double* q;
     const cd* pv;
     double dv, cv, gs;
     long long rec;
 
-    // by the whole warp; the shared memory is the warp's own
+    // by the whole team, lane its thread's index; the shared memory is its own
     __device__ void init(const GCtx& c, long long s, double gscale, GFastSmem* smem, int lane)
     {
         const TermRecs& R = c.R;
@@ -1865,9 +1883,9 @@ struct GFast {
         gs = gscale;
         m = R.m[s];
         phc = R.phc[s];
-        on = S != nullptr && phc <= kFastRows;
+        on = W > 1 && phc <= kFastRows;
         if (!on) return;
-        __syncwarp();  // the last record's cells are done
+        team_sync<W>();  // the last record's cells are done
         child = R.flags[s] & kFlagNewChild;
         hof = R.horthog[s];
         q = R.q + s * c.MC;
@@ -1879,14 +1897,14 @@ struct GFast {
         pv = c.Told.vals + c.P.tab_off[fam];
         const int pcnt = c.P.tab_cnt[fam];
         const int words = (1 << (phc - 1)) > 32 ? (1 << (phc - 1)) / 32 : 1;
-        for (int k = lane; k < words; k += 32) S->bits[k] = 0;
-        __syncwarp();
-        for (int k = lane; k < pcnt; k += 32) atomicOr(&S->bits[pk[k] >> 5], 1u << (pk[k] & 31));
+        for (int k = lane; k < words; k += kTeam) S->bits[k] = 0;
+        team_sync<W>();
+        for (int k = lane; k < pcnt; k += kTeam) atomicOr(&S->bits[pk[k] >> 5], 1u << (pk[k] & 31));
         // lambda keys
         const int z = R.z[s];
         zbit = child && z < phc ? 1 << z : 0;
         int col = 0, cneg = 0;
-        if (child) {
+        if (child && lane < 32) {
             const signed char* cmap = R.cmap + s * c.MC;
             const signed char* csmap = R.csmap + s * c.MC;
             const bool hc = R.flags[s] & kFlagHasCmap;
@@ -1897,46 +1915,48 @@ struct GFast {
                 if (hc && csmap[l] < 0) cneg |= 1 << k;
             }
         }
-        c0 = cneg;
+        if (lane == 0) S->c0 = cneg;
         if (lane < m) S->col[lane] = col;
         // partial sums of the low rows
         low = m < kFastLow ? m : kFastLow;
         if (lane == 0) S->T[0] = 0.0;
         for (int k = 0; k < low; k++) {
-            __syncwarp();
+            team_sync<W>();
             if ((hof >> k) & 1u) {
-                for (int i = lane; i < (1 << k); i += 32) S->T[i | (1 << k)] = S->T[i];
+                for (int i = lane; i < (1 << k); i += kTeam) S->T[i | (1 << k)] = S->T[i];
             } else {
                 const double qk = q[k];
-                for (int i = lane; i < (1 << k); i += 32) {
+                for (int i = lane; i < (1 << k); i += kTeam) {
                     const double t = S->T[i];
                     S->T[i | (1 << k)] = t - qk;
                     S->T[i] = t + qk;
                 }
             }
         }
-        __syncwarp();
-        // keys before each word
-        const int per = (words + 31) / 32;
-        int mine = 0;
-        for (int i = 0; i < per; i++) {
-            const int k = lane * per + i;
-            if (k < words) mine += __popc(S->bits[k]);
-        }
-        int pre = mine;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(kFull, pre, o);
-            if (lane >= o) pre += y;
-        }
-        pre -= mine;
-        for (int i = 0; i < per; i++) {
-            const int k = lane * per + i;
-            if (k < words) {
-                S->pref[k] = (unsigned short)pre;
-                pre += __popc(S->bits[k]);
+        team_sync<W>();
+        // keys before each word, by the first warp
+        if (lane < 32) {
+            const int per = (words + 31) / 32;
+            int mine = 0;
+            for (int i = 0; i < per; i++) {
+                const int k = lane * per + i;
+                if (k < words) mine += __popc(S->bits[k]);
+            }
+            int pre = mine;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(kFull, pre, o);
+                if (lane >= o) pre += y;
+            }
+            pre -= mine;
+            for (int i = 0; i < per; i++) {
+                const int k = lane * per + i;
+                if (k < words) {
+                    S->pref[k] = (unsigned short)pre;
+                    pre += __popc(S->bits[k]);
+                }
             }
         }
-        __syncwarp();
+        team_sync<W>();
     }
     __device__ cd look(int enc) const
     {
@@ -1955,7 +1975,7 @@ struct GFast {
             if (!(hof & (1u << k))) ygi += ((key >> k) & 1) ? -q[k] : q[k];
         int lp;
         if (child) {
-            lp = c0;
+            lp = S->c0;
             for (int b = 0; b < m; b++) lp ^= -((key >> b) & 1) & S->col[b];
         } else {
             lp = key & ((1 << phc) - 1);
@@ -2105,9 +2125,9 @@ template <int D>
 __global__ void k_gtable_prep(GCtx c, const int* roots_list, long long nroots, const int* gcnt, const long long* goff,
                               const int* members, const long long* toff, Tables Tnew, int* gnr, int* gitems,
                               int* gcells, int* minfo, double* rps2, double* mps2, int* rflag, int* mflag,
-                              int* pr_mcnt, int* pr_cells, int* pr_items, int* need, int* over)
+                              int* pr_mcnt, int* pr_cells, int* pr_items, int* need, int* over, long long* big)
 {
-    extern __shared__ unsigned smem_g[];
+    extern __shared__ __align__(16) unsigned smem_g[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwb = blockDim.x >> 5;
     const int MC = c.MC;
     const int words = (1 << MC) > 32 ? (1 << MC) / 32 : 1;
@@ -2149,6 +2169,7 @@ __global__ void k_gtable_prep(GCtx c, const int* roots_list, long long nroots, c
             rps2[ri] = R.ps2[r];
             rflag[ri] = 0;
             pr_mcnt[ri] = pr_cells[ri] = pr_items[ri] = 0;
+            if (nR > kFlatMaxCells) big[atomicAdd(over + 2, 1)] = ri;  // (in any order: each is by itself)
         }
         const long long mb = goff[r];
         for (int j = lane; j < nmem; j += 32) {
@@ -2285,35 +2306,59 @@ __global__ void k_gtable_combine(GCtx c, const int* roots_list, long long nroots
     }
 }
 
-template <int D>
-__global__ void k_gtable(GCtx c, const int* roots_list, long long nroots, const int* gcnt, const long long* goff,
-                         const int* members, const double* gscale_e, const long long* toff, Tables Tnew, int* tcnt,
-                         int* alive, int* src, cd* scratch, long long scratch_per_warp, const int* rflag,
-                         const int* gnr, int* pr_root, int* pr_mb, int* pr_mcnt, int* pr_cells, int* pr_items,
-                         int* err)
+// A group per team of W warps: a warp for the groups of at most kFlatMaxCells
+// cells (and all of them where the bitmaps are in global memory), a block of
+// kBigWarps for the larger ones the preparation listed (big, nbig; one after
+// another from a counter).  Members come one after another either way, each
+// member's cells side by side; an own-table member's values are kept in the
+// scratch for the sums, and the orientations are the preparation's.
+// Bound by latency (at a warp a group and 126 registers the FP64 pipe was 32 %
+// busy, 16 warps an SM), so small teams and enough blocks: 5-state sliding
+// windows, ms a pass by warps x blocks an SM: 8 x 2 245, 4 x 4 233, 8 x 3 230,
+// 4 x 6 225, 4 x 7 and 4 x 8 223, 2 x 16 233; 264 with a warp a group and the
+// masks and own values computed again.
+constexpr int kBigWarps = 4, kBigBlocks = 7;
+
+template <int D, int W>
+__global__ void __launch_bounds__(W == 1 ? 128 : 32 * W, W == 1 ? 1 : kBigBlocks)
+k_gtable(GCtx c, const int* roots_list, long long nroots, const int* gcnt, const long long* goff, const int* members,
+         const double* gscale_e, const long long* toff, Tables Tnew, int* tcnt, int* alive, int* src, cd* scratch,
+         long long scratch_per_warp, const int* rflag, const int* gnr, int* pr_root, int* pr_mb, int* pr_mcnt,
+         int* pr_cells, int* pr_items, int* err, const int* minfo, const long long* big, long long nbig, int* ticket)
 {
-    extern __shared__ unsigned smem_g[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwb = blockDim.x >> 5;
+    extern __shared__ __align__(16) unsigned smem_g[];
+    constexpr int kTeam = 32 * W;
+    // lane: this thread's index in its team; wl: in its warp
+    const int wl = threadIdx.x & 31, lane = W == 1 ? wl : threadIdx.x;
+    const int wib = W == 1 ? threadIdx.x >> 5 : 0, nwb = W == 1 ? blockDim.x >> 5 : 1;
+    const bool first_warp = W == 1 || threadIdx.x < 32;
+    __shared__ int s_int[2];
     const int MC = c.MC;
     const int words = (1 << MC) > 32 ? (1 << MC) / 32 : 1;
     const int capMC = c.capR;
-    const size_t pw = (size_t)(3 * words + 32 + capMC);
+    const size_t pw = (size_t)(2 * words + 32 + capMC);
     unsigned* PB = c.gbits ? c.gbits + (size_t)((long long)blockIdx.x * nwb + wib) * pw : smem_g + (size_t)wib * pw;
     unsigned* RK = PB + words;
-    unsigned* OK = RK + words;
-    int* bmk = reinterpret_cast<int*>(OK + words);
+    int* bmk = reinterpret_cast<int*>(RK + words);
     int* RKL = bmk + 32;
-    // after the warps' bitmaps; none where those are in global memory
-    GFastSmem* fast = nullptr;
-    if (!c.gbits) {
-        const size_t at = (pw * nwb * sizeof(unsigned) + 15) & ~(size_t)15;
-        fast = reinterpret_cast<GFastSmem*>(reinterpret_cast<char*>(smem_g) + at) + wib;
-    }
-    GFast<D> gf;
+    // a block's, after its bitmaps (see GFast)
+    GFastSmem* fast =
+        W > 1 ? reinterpret_cast<GFastSmem*>(smem_g + ((pw + 3) & ~(size_t)3)) : nullptr;
+    GFast<D, W> gf;
     const long long gw = (long long)blockIdx.x * nwb + wib;
     cd* scr = scratch + gw * scratch_per_warp;
     const TermRecs& R = c.R;
-    for (long long ri = gw; ri < nroots; ri += (long long)gridDim.x * nwb) {
+    for (long long ri = gw;; ri += (long long)gridDim.x * nwb) {
+        if (W > 1) {
+            // the next large group
+            __syncthreads();
+            if (threadIdx.x == 0) s_int[0] = atomicAdd(ticket, 1);
+            __syncthreads();
+            if (s_int[0] >= nbig) break;
+            ri = big[s_int[0]];
+        }
+        if (W == 1 && ri >= nroots) break;
+        if (W == 1 && nbig && gnr[ri] > kFlatMaxCells) continue;
         if (rflag[ri]) continue;  // kept root: k_gtable_combine
         // the root is approximated out (or has no cells): the serial path
         const long long r = roots_list[ri];
@@ -2337,10 +2382,15 @@ __global__ void k_gtable(GCtx c, const int* roots_list, long long nroots, const 
         int* okeys = Tnew.keys + out_off;
         cd* ovals = Tnew.vals + out_off;
         // ---- root cells
-        if (R.flags[r] & kFlagNewChild) new_child_cells<D>(c, r, RK, PB, bmk, lane);
-        else own_cells<D>(c, r, RK, lane);
-        int nR = bm_extract(RK, m, RKL, capMC, lane);
-        __syncwarp();
+        int nR = 0;
+        if (first_warp) {
+            if (R.flags[r] & kFlagNewChild) new_child_cells<D>(c, r, RK, PB, bmk, wl);
+            else own_cells<D>(c, r, RK, wl);
+            nR = bm_extract(RK, m, RKL, capMC, wl);
+        }
+        if (W > 1 && lane == 0) s_int[1] = nR;
+        team_sync<W>();
+        if (W > 1) nR = s_int[1];
         if (nR > cap || nR > capMC) {
             if (lane == 0) set_err(err, kErrRootCellsOverflow);
             nR = cap < capMC ? cap : capMC;
@@ -2352,13 +2402,13 @@ __global__ void k_gtable(GCtx c, const int* roots_list, long long nroots, const 
         if (!root_out) {
             const double ps2 = R.ps2[root];
             gf.init(c, root, gs, fast, lane);
-            for (int k = lane; k < nR; k += 32) {
+            for (int k = lane; k < nR; k += kTeam) {
                 const cd v = gf.cell(c, RKL[k]);
                 okeys[k] = RKL[k];
                 ovals[k] = v;
                 if (above_approx_threshold(ps2, v.re, v.im)) negl = false;
             }
-            negl = __all_sync(kFull, negl);
+            negl = team_all<W>(negl);
         }
         const int nmem = gcnt[r];
         const int* mem = members + goff[r];
@@ -2371,27 +2421,30 @@ __global__ void k_gtable(GCtx c, const int* roots_list, long long nroots, const 
             long long alfr = r;
             while (kidx < nmem) {
                 const long long cm = mem[kidx++];
-                if (R.flags[cm] & kFlagNewChild) {
+                if (!first_warp) {
+                } else if (R.flags[cm] & kFlagNewChild) {
                     int sg = 0;
-                    if (lane == 0) {
+                    if (wl == 0) {
                         sg = orientation_mask<D>(R.A + alfr * MC * D, R.A + cm * MC * D, m);
                         if (sg & top) sg ^= rev;
                     }
                     sg = __shfl_sync(kFull, sg, 0);
                     // re-orient the group's cell list into RK and re-sort
-                    for (int k = lane; k < words; k += 32) RK[k] = 0;
+                    for (int k = wl; k < words; k += 32) RK[k] = 0;
                     __syncwarp();
-                    for (int k = lane; k < nR; k += 32) {
+                    for (int k = wl; k < nR; k += 32) {
                         const int key = RKL[k] ^ sg;
                         if (key >= 0 && key < (1 << m)) atomicOr(&RK[key >> 5], 1u << (key & 31));
                     }
                     __syncwarp();
-                    nR = bm_extract(RK, m, RKL, capMC, lane);
+                    nR = bm_extract(RK, m, RKL, capMC, wl);
                 } else {
-                    own_cells<D>(c, cm, RK, lane);
-                    nR = bm_extract(RK, m, RKL, capMC, lane);
+                    own_cells<D>(c, cm, RK, wl);
+                    nR = bm_extract(RK, m, RKL, capMC, wl);
                 }
-                __syncwarp();
+                if (W > 1 && lane == 0) s_int[1] = nR;
+                team_sync<W>();
+                if (W > 1) nR = s_int[1];
                 if (nR > cap) {
                     if (lane == 0) set_err(err, kErrMemberCellsOverflow);
                     nR = cap;
@@ -2399,13 +2452,13 @@ __global__ void k_gtable(GCtx c, const int* roots_list, long long nroots, const 
                 const double ps2c = R.ps2[cm];
                 bool ng = true;
                 gf.init(c, cm, gs, fast, lane);
-                for (int k = lane; k < nR; k += 32) {
+                for (int k = lane; k < nR; k += kTeam) {
                     const cd v = gf.cell(c, RKL[k]);
                     okeys[k] = RKL[k];
                     ovals[k] = v;
                     if (above_approx_threshold(ps2c, v.re, v.im)) ng = false;
                 }
-                ng = __all_sync(kFull, ng);
+                ng = team_all<W>(ng);
                 if (!ng) {
                     root = cm;
                     break;
@@ -2418,7 +2471,7 @@ __global__ void k_gtable(GCtx c, const int* roots_list, long long nroots, const 
                 alive[r] = 0;
                 tcnt[r] = 0;
             }
-            __syncwarp();
+            team_sync<W>();
             continue;
         }
         // RK holds the root's cells as a bitmap, RKL as a sorted list.
@@ -2436,31 +2489,37 @@ __global__ void k_gtable(GCtx c, const int* roots_list, long long nroots, const 
                 tcnt[r] = nR;
                 src[r] = (int)root;
             }
-            __syncwarp();
+            team_sync<W>();
             continue;
         }
         // ---- members: make_gtable + add_gtables (flattening.hpp:493-552)
         for (; kidx < nmem; kidx++) {
             const long long cm = mem[kidx];
-            const bool newc = R.flags[cm] & kFlagNewChild;
-            bool own = false;
-            if (!newc) own = c.P.B_cnt[R.fam[cm]] == nR;
+            bool own;
             int sig = 0;
-            if (lane == 0) sig = orientation_mask<D>(R.A + root * MC * D, R.A + cm * MC * D, m);
-            sig = __shfl_sync(kFull, sig, 0);
+            if (root == r) {
+                const int info = minfo[goff[r] + kidx];
+                sig = info & ~kInfoOwn;
+                own = info & kInfoOwn;
+            } else {
+                own = !(R.flags[cm] & kFlagNewChild) && c.P.B_cnt[R.fam[cm]] == nR;
+                // (every warp its own copy: it takes no longer than waiting for one)
+                if (wl == 0) sig = orientation_mask<D>(R.A + root * MC * D, R.A + cm * MC * D, m);
+                sig = __shfl_sync(kFull, sig, 0);
+            }
             const int sigf = (sig & top) ? (sig ^ rev) : sig;
             const double ps2c = R.ps2[cm];
             bool ng = true;
             gf.init(c, cm, gs, fast, lane);
             if (!own) {
-                for (int k = lane; k < nR; k += 32) {
+                for (int k = lane; k < nR; k += kTeam) {
                     const cd v = gf.cell(c, RKL[k] ^ sigf);
                     scr[k] = v;
                     if (above_approx_threshold(ps2c, v.re, v.im)) ng = false;
                 }
-                ng = __all_sync(kFull, ng);
+                ng = team_all<W>(ng);
                 if (!ng)
-                    for (int k = lane; k < nR; k += 32) {
+                    for (int k = lane; k < nR; k += kTeam) {
                         const int bi = RKL[k];
                         const int t = bi ^ sig;
                         const bool cj = t & top;
@@ -2473,35 +2532,36 @@ __global__ void k_gtable(GCtx c, const int* roots_list, long long nroots, const 
                         ovals[k] = cadd(a, cj ? cconj(v) : v);
                     }
             } else {
-                own_cells<D>(c, cm, OK, lane);
                 const int fam = R.fam[cm];
                 const int* B = c.Bkeys + c.P.B_off[fam];
-                const int n = c.P.B_cnt[fam];
-                for (int k = lane; k < n; k += 32) {
+                const int n = c.P.B_cnt[fam], flip = c.P.bflip[fam];
+                for (int k = lane; k < n; k += kTeam) {
                     const cd v = gf.cell(c, B[k]);
+                    scr[k] = v;
                     if (above_approx_threshold(ps2c, v.re, v.im)) ng = false;
                 }
-                ng = __all_sync(kFull, ng);
+                ng = team_all<W>(ng);
                 if (!ng)
-                    for (int k = lane; k < nR; k += 32) {
+                    for (int k = lane; k < nR; k += kTeam) {
                         const int bi = RKL[k];
                         const int t = bi ^ sig;
                         const bool cj = t & top;
                         const int bj = cj ? (t ^ rev) : t;
-                        if (bj < 0 || bj >= (1 << m) || !bm_get(OK, bj)) continue;
-                        const cd v = gf.cell(c, bj);
+                        const int at = bj < (1 << m) ? bsearch_key_xor(B, n, bj, flip) : -1;
+                        if (at < 0) continue;
+                        const cd v = scr[at];
                         const cd a = ovals[k];
                         ovals[k] = cadd(a, cj ? cconj(v) : v);
                     }
             }
-            __syncwarp();
+            team_sync<W>();
         }
         if (lane == 0) {
             alive[r] = 1;
             tcnt[r] = nR;
             src[r] = (int)root;
         }
-        __syncwarp();
+        team_sync<W>();
     }
 }
 
@@ -3123,35 +3183,46 @@ void Kernels<D>::ftr_graph_destroy(void* gv)
 static inline size_t gtable_smem_per_warp(int MC, int capR)
 {
     const int words = (1 << MC) > 32 ? (1 << MC) / 32 : 1;
-    return (size_t)(3 * words + 32 + capR) * 4;
+    return (size_t)(2 * words + 32 + capR) * 4;
 }
 
 template <int D>
 void Kernels<D>::gtable(TermRecs R, const int* roots_list, long long nroots, const int* gcnt, const long long* goff,
                         const int* members, ParentList P, Tables Told, const int* Bkeys, const double* gscale,
                         const long long* toff, Tables Tnew, int* tcnt, int* alive, int* src, cd* scratch,
-                        long long scratch_per_warp, const GFlat& f, int MC, int* err, const LaunchCfg& c,
-                        long long max_warps)
+                        long long scratch_per_warp, const GFlat& f, int MC, int* err, long long nbig, int* ticket,
+                        const LaunchCfg& c, long long max_warps)
 {
     if (nroots == 0) return;
     const bool global_bits = MC > kSmemBitmapRows && c.gbits;
     GCtx ctx{R, P, Told, Bkeys, MC, global_bits ? c.gbits : nullptr, cells_cap_of(c, MC, D)};
     const size_t pw = gtable_smem_per_warp(MC, ctx.capR);
-    int warps = global_bits ? 4 : (int)(96 * 1024 / (pw + sizeof(GFastSmem)));
+    int warps = global_bits ? 4 : (int)(96 * 1024 / pw);
     if (warps > 4) warps = 4;
     if (warps < 1) warps = 1;
-    const size_t sm = global_bits ? 0 : ((pw * warps + 15) & ~(size_t)15) + sizeof(GFastSmem) * warps;
-    if (!global_bits) cudaFuncSetAttribute(k_gtable<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const size_t sm = global_bits ? 0 : pw * warps;
+    if (!global_bits)
+        cudaFuncSetAttribute(k_gtable<D, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     int grid = grid_for(nroots, warps, c.num_sms, 16);
     if (global_bits && (long long)grid * warps > c.gbits_warps) grid = (int)(c.gbits_warps / warps);
     // a scratch region sized for max_warps warps (the caller guarantees
     // max_warps >= 4 >= warps): the warps stride over the roots, so fewer of
     // them give the same tables
     if (max_warps > 0 && (long long)grid * warps > max_warps) grid = (int)(max_warps / warps);
+    if (global_bits) nbig = 0;
     ++g_launches;
-    k_gtable<D><<<grid, warps * 32, sm, c.stream>>>(ctx, roots_list, nroots, gcnt, goff, members, gscale, toff, Tnew,
-                                                    tcnt, alive, src, scratch, scratch_per_warp, f.rflag, f.gnr,
-                                                    f.pr_root, f.pr_mb, f.pr_mcnt, f.pr_cells, f.pr_items, err);
+    k_gtable<D, 1><<<grid, warps * 32, sm, c.stream>>>(
+        ctx, roots_list, nroots, gcnt, goff, members, gscale, toff, Tnew, tcnt, alive, src, scratch, scratch_per_warp,
+        f.rflag, f.gnr, f.pr_root, f.pr_mb, f.pr_mcnt, f.pr_cells, f.pr_items, err, f.minfo, nullptr, nbig, nullptr);
+    if (nbig == 0) return;
+    const size_t smb = ((pw + 15) & ~(size_t)15) + sizeof(GFastSmem);
+    cudaFuncSetAttribute(k_gtable<D, kBigWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb);
+    int gb = grid_for(nbig, 1, c.num_sms, kBigBlocks);
+    if (max_warps > 0 && gb > max_warps) gb = (int)max_warps;
+    ++g_launches;
+    k_gtable<D, kBigWarps><<<gb, 32 * kBigWarps, smb, c.stream>>>(
+        ctx, roots_list, nroots, gcnt, goff, members, gscale, toff, Tnew, tcnt, alive, src, scratch, scratch_per_warp,
+        f.rflag, f.gnr, f.pr_root, f.pr_mb, f.pr_mcnt, f.pr_cells, f.pr_items, err, f.minfo, f.pr_moff, nbig, ticket);
 }
 
 template <int D>
@@ -3194,7 +3265,7 @@ void Kernels<D>::gtable_prep(TermRecs R, const int* roots_list, long long nroots
     ++g_launches;
     k_gtable_prep<D><<<grid, warps * 32, sm, c.stream>>>(
         ctx, roots_list, nroots, gcnt, goff, members, toff, Tnew, f.gnr, gitems, gcells, f.minfo, f.rps2, f.mps2,
-        f.rflag, f.mflag, f.pr_mcnt, f.pr_cells, f.pr_items, need, over);
+        f.rflag, f.mflag, f.pr_mcnt, f.pr_cells, f.pr_items, need, over, f.pr_moff);
 }
 
 template <int D>

@@ -65,7 +65,7 @@ inline int cells_cap_of(const LaunchCfg& c, int MC, int D)
 inline long long gtable_bitmap_words(int MC, int D, int cells_cap = 0)
 {
     const long long words = (1LL << MC) > 32 ? (1LL << MC) / 32 : 1;
-    return 3 * words + 32 + (cells_cap > 0 ? cells_cap : half_cells_cap(MC, D));
+    return 2 * words + 32 + (cells_cap > 0 ? cells_cap : half_cells_cap(MC, D));
 }
 
 // N-D conditional pdf (csrc/mce_ndpdf.cu): one estimator's terms (a
@@ -240,12 +240,14 @@ struct Kernels {
                                 int* resume, int max_rounds, int* err, const LaunchCfg& c);
     static void ftr_graph_collect(void* graph);
     static void ftr_graph_destroy(void* graph);
-    // g-tables of every reduction group (flattening.hpp:318-568).
+    // g-tables of every reduction group (flattening.hpp:318-568).  nbig: the
+    // groups of many cells the preparation listed in GFlat::pr_moff (which the
+    // promoted-root pass fills only later); ticket: a zeroed counter.
     static void gtable(TermRecs R, const int* roots_list, long long nroots, const int* gcnt,
                        const long long* goff, const int* members, ParentList P, Tables Told, const int* Bkeys,
                        const double* gscale, const long long* toff, Tables Tnew, int* tcnt, int* alive,
                        int* src, cd* scratch, long long scratch_per_warp, const GFlat& f, int MC, int* err,
-                       const LaunchCfg& c, long long max_warps = 0);
+                       long long nbig, int* ticket, const LaunchCfg& c, long long max_warps = 0);
     // the members left after promotions (GFlat::pr_*), a flat pass
     static void gtable_promoted(TermRecs R, const int* roots_list, long long nroots, long long nmem,
                                 long long nitems, long long ncells, const int* members, ParentList P, Tables Told,
