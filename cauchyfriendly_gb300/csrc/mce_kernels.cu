@@ -688,6 +688,18 @@ __global__ void k_tp(ParentList P, long long nP, const EstStep<D>* st, int with_
 // sign vector, written to vsv (-1: skipped).  Most parents have few subsets
 // (a 3-state term of 4-6 hyperplanes has 4-20), so one parent per warp would
 // leave most lanes idle; here every lane solves a subset.
+// Bound by the FP64 pipe, so only what the factorisation and the solve need
+// goes there: the norm is bounded and the rows' signs are found in single
+// precision, and computed as the reference does only where that does not
+// settle them (see kSignRel).
+// A row's sum in single precision from operands cut to 24 bits is off by less
+// than (2 + (D + 2) / 2) 2^-23 of the sum of its terms' magnitudes, and by D
+// 2^-65 for operands below the single-precision range when the others are
+// below 2^60; beyond four times that its sign is that of the FP64 sum.
+// 5-state sliding windows 51 -> 41 ms a pass, 4,096 3-state estimators 13.2 ->
+// 9.6 ms.
+constexpr float kSignRel = 4e-6f, kSignAbs = 8.7e-19f;
+constexpr unsigned kSignMaxHi = (1023u + 60u) << 20;
 template <int D>
 __global__ void k_build_B_vertices(ParentList P, long long nP, const long long* voff, long long nv,
                                    const double* bpert_all, int MC, const int* combo_off,
@@ -717,28 +729,61 @@ __global__ void k_build_B_vertices(ParentList P, long long nP, const long long* 
         // the exact LU factors settles the well-conditioned subsets; the
         // reference's explicit-inverse value is computed only when the bound is
         // not at least ten times below 1e12.
-        double nrm = -1;
+        float nrm_up = 0.f;
         for (int cc = 0; cc < D; cc++) {
-            double sm = 0;
-            for (int r = 0; r < D; r++) sm += fabs(Ac[r * D + cc]);
-            if (dlt(nrm, sm)) nrm = sm;
+            float sm = 0.f;
+            for (int r = 0; r < D; r++) sm += abs32(Ac[r * D + cc], true);
+            nrm_up = fmaxf(nrm_up, sm);
         }
         if (plu<D>(Ac, v, perm, piv)) {
-            const double bound = nrm * (double)inv_norm1_bound<D>(Ac);
-            if ((bound <= 0.1 * kCondEps) || !cond1_exceeds<D>(Ac, piv, perm, nrm, kCondEps)) {
+            bool cond_ok = nrm_up * inv_norm1_bound<D>(Ac) <= (float)(0.099 * kCondEps);
+            if (!cond_ok) {
+                double nrm = -1;
+                for (int cc = 0; cc < D; cc++) {
+                    double sm = 0;
+                    for (int r = 0; r < D; r++) sm += fabs(As[c[r] * D + cc]);
+                    if (dlt(nrm, sm)) nrm = sm;
+                }
+                cond_ok = !cond1_exceeds<D>(Ac, piv, perm, nrm, kCondEps);
+            }
+            if (cond_ok) {
                 lu_solve_inplace<D>(Ac, piv, v);
-                unsigned inmask = 0;
-                for (int j = 0; j < D; j++) inmask |= 1u << c[j];
+                unsigned rows = (1u << m) - 1;
+                for (int j = 0; j < D; j++) rows &= ~(1u << c[j]);
+                float vf[D];
+                unsigned vbig = 0;
+                for (int j = 0; j < D; j++) {
+                    vf[j] = trunc32(v[j]);
+                    vbig = max(vbig, (unsigned)__double2hiint(v[j]) & 0x7fffffffu);
+                }
                 int niv = 0;
+                unsigned open = 0;
                 // the m - D rows outside the subset, every lane on one of its
-                // own rows per iteration (no idle lanes in the FP64 work)
-                int a = 0;
-                for (int q = 0; q < m - D; q++) {
-                    while ((inmask >> a) & 1u) a++;
+                // own rows per iteration
+                for (; rows; rows &= rows - 1) {
+                    const int a = __ffs(rows) - 1;
+                    const double b = bp[a];
+                    const float bf = trunc32(b);
+                    unsigned big = max(vbig, (unsigned)__double2hiint(b) & 0x7fffffffu);
+                    float s = -bf, mag = fabsf(bf);
+                    for (int j = 0; j < D; j++) {
+                        const double Aj = As[a * D + j];
+                        const float Af = trunc32(Aj);
+                        big = max(big, (unsigned)__double2hiint(Aj) & 0x7fffffffu);
+                        s = __fmaf_rn(Af, vf[j], s);
+                        mag = __fmaf_rn(fabsf(Af), fabsf(vf[j]), mag);
+                    }
+                    if (big < kSignMaxHi && fabsf(s) > __fmaf_rn(kSignRel, mag, kSignAbs)) {
+                        if (s < 0.f) niv |= 1 << a;
+                    } else {
+                        open |= 1u << a;
+                    }
+                }
+                for (; open; open &= open - 1) {
+                    const int a = __ffs(open) - 1;
                     double s = 0.0;
-                    for (int j = 0; j < D; j++) s += lu_mul<D>(As[a * D + j], v[j]);
+                    for (int j = 0; j < D; j++) s += As[a * D + j] * v[j];
                     if (neg(s - bp[a])) niv |= 1 << a;
-                    a++;
                 }
                 out = niv;
             }

@@ -431,3 +431,25 @@ def test_table_cells_at_the_largest_parents_of_the_shared_memory_path(states, up
     gpu.close()
     orc.close()
     G.compare_records(got, want, check_terms=False)
+
+
+@pytest.mark.parametrize("states,updates", [(3, 7), (5, 6)])
+@pytest.mark.parametrize("exponent", [58, 66, -58, -140])
+def test_vertex_signs_do_not_depend_on_the_perturbation_scale(states, updates, exponent):
+    """A perturbation scaled by a power of two scales every vertex exactly and
+    leaves the cells alone: within single precision's range, beyond the limit
+    of its row signs (2^60), and below its smallest number, where the signs
+    are computed in double precision, the steps are the same bit for bit."""
+    from cauchyfriendly_gb300 import workloads as W
+    prob = W.three_state_lti(seed=6, steps=8) if states == 3 else W.five_state_ltv_windows(seed=1, steps=8)
+    rp, bp = oracle.draw_reference_constants(21, states, oracle.max_shape_of(prob))
+    ests = [_GpuAdapter(prob, rp, np.asarray(bp) * f) for f in (1.0, 2.0 ** exponent)]
+    for i in range(updates):
+        errs = [est.step(i // prob["p"], i % prob["p"]) for est in ests]
+        assert errs[0] == errs[1]
+        assert ests[0].num_terms() == ests[1].num_terms()
+        a, b = (est.moments() for est in ests)
+        for key in ("raw_fz", "raw_mean", "raw_cov"):
+            assert G.bitwise_equal(np.atleast_1d(a[key]), np.atleast_1d(b[key])), (i, key)
+    for est in ests:
+        est.close()
