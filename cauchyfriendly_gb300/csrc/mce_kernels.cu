@@ -2158,9 +2158,10 @@ __device__ inline void own_cells(const GCtx& c, long long s, unsigned* bm, int l
 //                  each member's orientation and mode, the p sums;
 //   k_gtable_eval  (a thread per (term, cell) of every group)  g_cell, and
 //                  the term-approximation flags;
-//   k_gtable       (a warp per group)  the sums in member order; a group whose
-//                  root is approximated out takes the serial path, which
-//                  re-derives everything in the reference's order.
+//   k_gtable       (a warp per group, four for more than 64 cells)  the sums in
+//                  member order; a group whose root is approximated out takes
+//                  this path, which re-derives everything in the reference's
+//                  order.
 // Member info word: bits 0-15 the orientation mask relative to the root,
 // bit 30 the own-table mode.
 constexpr int kInfoOwn = 1 << 30;
@@ -2204,8 +2205,8 @@ __global__ void k_gtable_prep(GCtx c, const int* roots_list, long long nroots, c
         }
         for (int k = lane; k < nR; k += 32) okeys[k] = RKL[k];
         const int nmem = gcnt[r];
-        // groups of many cells fill warps on their own: they stay on the
-        // serial path, which keeps the items buffer small
+        // groups of many cells fill warps on their own: they are listed for
+        // k_gtable's teams, which keeps the items buffer small
         const bool flat = nR > 0 && nR <= kFlatMaxCells;
         if (lane == 0) {
             gnr[ri] = nR;
