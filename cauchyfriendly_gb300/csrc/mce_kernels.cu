@@ -2162,9 +2162,10 @@ __device__ inline void own_cells(const GCtx& c, long long s, unsigned* bm, int l
 //                  member order; a group whose root is approximated out takes
 //                  this path, which re-derives everything in the reference's
 //                  order.
-// Member info word: bits 0-15 the orientation mask relative to the root,
-// bit 30 the own-table mode.
+// Member info word: bit 30 the own-table mode, the bits below it the
+// orientation mask relative to the root, a bit per row.
 constexpr int kInfoOwn = 1 << 30;
+static_assert(kMaxBitmapRows <= 30, "an orientation bit per row below kInfoOwn");
 constexpr int kFlatMaxCells = 64;
 
 template <int D>
@@ -2274,7 +2275,7 @@ __global__ void k_gtable_eval(GCtx c, const int* roots_list, long long nroots, c
             } else {
                 const int m = R.m[r];
                 const int top = 1 << (m - 1), rev = (1 << m) - 1;
-                const int sig = info & 0xffff;
+                const int sig = info & ~kInfoOwn;
                 key = okeys[k] ^ ((sig & top) ? (sig ^ rev) : sig);
             }
             ps2 = mps2[mi];
@@ -2324,7 +2325,7 @@ __global__ void k_gtable_combine(GCtx c, const int* roots_list, long long nroots
         for (int j = 0; j < nmem; j++) {
             if (!mflag[mb + j]) continue;
             const int info = minfo[mb + j];
-            const int sig = info & 0xffff;
+            const int sig = info & ~kInfoOwn;
             const int sigf = (sig & top) ? (sig ^ rev) : sig;
             const int t = bi ^ sig;
             const bool cj = t & top;
@@ -2670,7 +2671,7 @@ __global__ void k_gtable_prom_eval(GCtx c, const int* roots_list, long long nroo
         } else {
             const int m = R.m[r];
             const int top = 1 << (m - 1), rev = (1 << m) - 1;
-            const int sig = info & 0xffff;
+            const int sig = info & ~kInfoOwn;
             key = Tnew.keys[toff[r] + k] ^ ((sig & top) ? (sig ^ rev) : sig);
         }
         const cd v = g_cell<D>(c, s, key, gscale_e[R.est[r]]);
@@ -2701,7 +2702,7 @@ __global__ void k_gtable_prom_combine(GCtx c, const int* roots_list, long long n
         for (int jj = 0; jj < nm; jj++) {
             if (!f.mflag[mb + jj]) continue;
             const int info = f.minfo[mb + jj];
-            const int sig = info & 0xffff;
+            const int sig = info & ~kInfoOwn;
             const int sigf = (sig & top) ? (sig ^ rev) : sig;
             const int t = bi ^ sig;
             const bool cj = t & top;

@@ -453,3 +453,39 @@ def test_vertex_signs_do_not_depend_on_the_perturbation_scale(states, updates, e
             assert G.bitwise_equal(np.atleast_1d(a[key]), np.atleast_1d(b[key])), (i, key)
     for est in ests:
         est.close()
+
+
+def test_flat_groups_of_more_than_sixteen_rows():
+    """Three states with eight noise columns and three measurements a step:
+    after the second measurement of the third step the reduction groups have
+    19 rows but at most 64 cells (all but one row lie in the plane orthogonal
+    to H), and their members differ in the signs of rows up to the 18th.  The
+    terms with their tables against the oracle's, and the moments of the
+    update after it."""
+    from cauchyfriendly_gb300 import workloads as W
+    prob = W.many_gamma(3, 8, 3, seed=0)
+    rng = np.random.Generator(np.random.PCG64(99))
+    prob["p"], prob["gamma"] = 3, np.array([0.2, 0.3, 0.3])
+    prob["H"] = np.vstack([prob["H"], rng.standard_normal((2, 3))])
+    prob["msmts"] = W.simulate(prob, rng)
+    rp, bp = oracle.draw_reference_constants(7, 3, oracle.max_shape_of(prob))
+    gpu = _GpuAdapter(prob, rp, bp)
+    orc = oracle.Oracle(prob, rp, bp)
+    got, want = [], []
+    for i in range(8):
+        for est, out in ((gpu, got), (orc, want)):
+            err = est.step(i // 3, i % 3)
+            rec = est.moments()
+            rec["err"] = int(err)
+            rec["Nt"] = est.num_terms()
+            rec["tps"] = est.terms_per_shape()
+            out.append(rec)
+    a, b = gpu.dump_terms(19), orc.dump_terms(19)
+    assert gpu.est.device_errors() == 0
+    gpu.close()
+    orc.close()
+    G.compare_records(got, want, check_terms=False)
+    assert b["shape"].max() == 19
+    assert np.array_equal(a["shape"], b["shape"]) and np.array_equal(a["cells"], b["cells"])
+    assert np.array_equal(a["keys"], b["keys"])
+    assert G.relerr(a["g"], b["g"]) <= G.REL_TOL, G.relerr(a["g"], b["g"])
