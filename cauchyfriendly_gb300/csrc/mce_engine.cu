@@ -843,6 +843,8 @@ public:
         s |= scan_tmp.ensure(1 << 16);
         s |= h_raw.ensure((size_t)E * (1 + D + D * D));
         s |= h_gscale.ensure(E);
+        // for the last updates, which a step that may not allocate can be too
+        s |= kall_est.ensure(E + 2);
         s |= h_tot.ensure(16);
         s |= h_ints.ensure(8);
         s |= h_hist.ensure((size_t)E * (MC + 1));
@@ -1394,7 +1396,6 @@ public:
         const int MCp = MC + 1;
         if (any_skip) {
             // terms after the MU per estimator (un-reduced count, cauchy_estimator.hpp:749-751, 806-812)
-            if ((s = kall_est.ensure(E + 2))) return s;
             pbeg(KID_SCAN);
             k_gather_bounds(kall_scan.ptr, E);
             pend();

@@ -165,3 +165,37 @@ def test_noalloc_step_matches_allocating_step(make):
     assert b.est.device_errors() == 0
     b.close()
 
+
+
+def _copies(n, steps):
+    """n copies of one estimator with one history."""
+    from cauchyfriendly_gb300 import workloads as W
+    q = W.three_state_lti(seed=3, steps=steps)
+    return [q] * n, [oracle.draw_reference_constants(31, 3, oracle.max_shape_of(q))] * n
+
+
+def test_noalloc_last_update_after_warming_the_others():
+    """A handle whose buffers were sized by the updates before the last one
+    only: a light last update, for which they suffice, is taken."""
+    _need_gpu()
+    probs, consts = _copies(8, 7)
+    b = _Batch(probs, consts)
+    H = b.H.copy()
+    for k in range(6):
+        assert b.call("mce_batch_step", k, 0)[0] == 0
+    b.est.reset()
+    for k in range(7):
+        # (rows orthogonal to H are not integrated: few terms)
+        b.H = H if k < 2 else H * 0.0
+        rc, _ = b.call("mce_batch_step_noalloc", k, 0)
+        assert rc == 0, (k, b.lib.load().mce_last_error())
+    light = [b.est.moments(i) for i in range(8)]
+    b.est.reset()
+    for k in range(7):
+        b.H = H if k < 2 else H * 0.0
+        assert b.call("mce_batch_step", k, 0)[0] == 0
+    for i, m in enumerate(light):
+        w = b.est.moments(i)
+        for key in ("raw_fz", "raw_mean", "raw_cov"):
+            assert G.bitwise_equal(np.atleast_1d(m[key]), np.atleast_1d(w[key])), (i, key)
+    b.close()
