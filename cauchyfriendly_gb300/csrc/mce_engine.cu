@@ -840,7 +840,7 @@ public:
         s |= gscale.ensure(E);
         s |= counters.ensure(8);
         s |= first_cnt.ensure(E + 1);
-        s |= scan_tmp.ensure(1 << 16);
+        s |= scan_tmp.ensure((size_t)kScanJobs << 16);  // scans of 2^27 values
         s |= h_raw.ensure((size_t)E * (1 + D + D * D));
         s |= h_gscale.ensure(E);
         // for the last updates, which a step that may not allocate can be too
@@ -1452,7 +1452,9 @@ public:
         if ((s = gfill.ensure(nR + 1))) return s;
         // the rounds' worklist counts and their long-list counts
         if ((s = ftr_cnt.ensure(2 * kFtrCntSlots))) return s;
-        const bool long_lists = nR >= kLongLists;
+        // (a step that may not allocate does without the list where no step
+        // before it was as large: the same reduction, its long buckets slower)
+        const bool long_lists = nR >= kLongLists && (!g_device_alloc_forbidden || (long long)ftr_long.cap > nR);
         if (long_lists && (s = ftr_long.ensure(nR + 1))) return s;
         if ((s = ensure_scan_scratch(std::max(nR, H) + 1))) return s;
         MCE_CUDA(cudaMemsetAsync(bcount.ptr, 0, sizeof(int) * 2 * H, lc.stream));

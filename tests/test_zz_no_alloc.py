@@ -199,3 +199,36 @@ def test_noalloc_last_update_after_warming_the_others():
         for key in ("raw_fz", "raw_mean", "raw_cov"):
             assert G.bitwise_equal(np.atleast_1d(m[key]), np.atleast_1d(w[key])), (i, key)
     b.close()
+
+
+def test_noalloc_steps_within_the_slack_of_the_buffers():
+    """Buffers that grew to half again their first size serve a somewhat
+    larger step than any before it, also past the 2^14 records from which long
+    buckets have a list of their own."""
+    _need_gpu()
+    n, steps = 100, 7
+    probs, consts = _copies(n, steps)
+    b = _Batch(probs, consts)
+    H = b.H.copy()
+
+    def go(fn_name, dense):
+        """`dense` of the estimators branch; the others' rows are orthogonal to H."""
+        b.est.reset()
+        b.H = H.copy()
+        b.H[dense:] = 0.0
+        for k in range(steps - 1):
+            rc, _ = b.call(fn_name, k, 0)
+            assert rc == 0, (fn_name, dense, k, b.lib.load().mce_last_error())
+        return [b.est.moments(i) for i in (0, dense - 1, n - 1)] + [[b.est.num_terms(i) for i in range(n)]]
+
+    # 556 records each in the sixth update: 15,085, 21,745 and 22,300
+    # (twice each: the terms are kept in two sets of buffers in turn)
+    for dense in (27, 27, 39, 39):
+        go("mce_batch_step", dense)
+    got = go("mce_batch_step_noalloc", 40)
+    want = go("mce_batch_step", 40)
+    assert got[3] == want[3]
+    for m, w in zip(got[:3], want[:3]):
+        for key in ("raw_fz", "raw_mean", "raw_cov"):
+            assert G.bitwise_equal(np.atleast_1d(m[key]), np.atleast_1d(w[key])), key
+    b.close()
