@@ -60,17 +60,18 @@ static void set_error(const std::string& s) { g_last_error = s; }
 // manager, 126 of 335 ms for a 5-state one.  The buffers come from a
 // stream-ordered pool of the library, one per device, which keeps at most a
 // 32nd of the device's memory between uses (the driver returns what is above
-// that at the next synchronisation), and kPoolKeepIdle bytes once no handle is
-// alive.  Inside a step (AllocOn) buffers are freed and allocated in the order
-// of the handle's stream, on which all of a step's work is queued or joined;
-// elsewhere an allocation is complete, and a freed buffer's work done, before
-// the call returns, as with cudaMalloc and cudaFree.
+// that at the next synchronisation), and kPoolKeepIdle bytes once no handle
+// and no relative system is alive.  Inside a step (AllocOn) buffers are freed
+// and allocated in the order of the handle's stream, on which all of a step's
+// work is queued or joined; elsewhere an allocation is complete, and a freed
+// buffer's work done, before the call returns, as with cudaMalloc and cudaFree.
 constexpr size_t kPoolKeepIdle = 256u << 20;
 extern thread_local cudaStream_t t_alloc_stream;  // of the step this thread is in, or null
 extern thread_local bool t_alloc_idle;            // the buffers being freed have no work left
 cudaError_t dev_malloc(void** p, size_t bytes);
 void dev_free(void* p);
-void pool_handles(int change);  // a handle was made (+1) or destroyed (-1)
+// A handle or a relative system is being made (+1) or is gone (-1).
+void pool_handles(int change);
 struct AllocOn {
     cudaStream_t prev;
     explicit AllocOn(cudaStream_t s) : prev(t_alloc_stream) { t_alloc_stream = s; }
@@ -2649,6 +2650,7 @@ mce_handle* mce_batch_create(int n_est, int d, int cmcc, int pncc, int p, const 
         b_pert = bps.data();
         stride = msmax;
     }
+    pool_handles(1);
     EngineBase* eng = nullptr;
 #define MCE_CASE(D)                                                                                    \
     case D:                                                                                            \
@@ -2660,12 +2662,15 @@ mce_handle* mce_batch_create(int n_est, int d, int cmcc, int pncc, int p, const 
     }
 #undef MCE_CASE
     if (st != MCE_OK) {
-        delete eng;
+        {
+            const AllocIdle idle;  // the destructor waits for the engine's streams first
+            delete eng;
+        }
+        pool_handles(-1);
         if (status) *status = st;
         return nullptr;
     }
     h = new mce_handle{eng};
-    pool_handles(1);
     if (status) *status = MCE_OK;
     return h;
 }
@@ -2871,11 +2876,12 @@ mce_rel2d* mce_rel2d_create(mce_handle* primary, int est_p, mce_handle* secondar
     int s = MCE_ERR_ARG;
     mce_rel2d* r = nullptr;
     if (!bad(primary, est_p) && !bad(secondary, est_s) && Trel && bar_nu_full) {
+        pool_handles(1);
         r = new mce_rel2d();
         s = rel2d_build(r, *primary->eng, est_p, *secondary->eng, est_s, Trel, bar_nu_full, full_solve,
                         with_term_approx, term_approx_eps, moments, counts);
         if (s != MCE_OK) {
-            delete r;
+            mce_rel2d_destroy(r);
             r = nullptr;
         }
     }
@@ -2894,8 +2900,12 @@ double mce_rel2d_device_ms(mce_rel2d* r, int which) { return r && which >= 0 && 
 long long mce_rel2d_launch_count(mce_rel2d* r) { return r ? r->launches : MCE_ERR_ARG; }
 void mce_rel2d_destroy(mce_rel2d* r)
 {
-    const AllocIdle idle;  // the destructor waits for the object's stream first
-    delete r;
+    if (!r) return;
+    {
+        const AllocIdle idle;  // the destructor waits for the object's stream first
+        delete r;
+    }
+    pool_handles(-1);
 }
 long long mce_post_mu_terms(mce_handle* h) { return h ? h->eng->post_mu_terms : MCE_ERR_ARG; }
 double mce_host_time_ms(mce_handle* h, int which) { return h && which >= 0 && which < 3 ? h->eng->host_ms[which] : -1.0; }

@@ -470,7 +470,8 @@ int mce_reset(mce_handle* h);
  * reference's terms are reallocated each step, include/cauchy_estimator.hpp)
  * while small windows keep theirs.  Released memory goes back to the
  * library's pool, which keeps at most a 32nd of the device's memory for its
- * handles' next buffers (256 MiB once no handle is alive). */
+ * handles' next buffers (256 MiB once no handle and no relative system is
+ * alive). */
 long long mce_trim_memory(mce_handle* h, long long min_bytes);
 /* reinitialize_start_statistics (include/cauchy_estimator.hpp:1302). */
 int mce_reinitialize_start_statistics(mce_handle* h, int est, const double* A0, const double* p0, const double* b0);
