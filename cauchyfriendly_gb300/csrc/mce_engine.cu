@@ -72,6 +72,7 @@ cudaError_t dev_malloc(void** p, size_t bytes);
 void dev_free(void* p);
 // A handle or a relative system is being made (+1) or is gone (-1).
 void pool_handles(int change);
+void pool_release();  // what the current device's pool holds unused goes back to the device
 struct AllocOn {
     cudaStream_t prev;
     explicit AllocOn(cudaStream_t s) : prev(t_alloc_stream) { t_alloc_stream = s; }
@@ -158,6 +159,12 @@ void dev_free(void* p)
     }
     if (!t_alloc_idle) cudaDeviceSynchronize();
     cudaFree(p);  // (of pool memory: no synchronisation of its own)
+}
+
+void pool_release()
+{
+    DevPool* d = device_pool();
+    if (d && d->pool) cudaMemPoolTrimTo(d->pool, 0);
 }
 
 void pool_handles(int change)
@@ -944,7 +951,11 @@ public:
         if (min_bytes > 0 && trim_pass(false) < min_bytes) return 0;
         drain();
         const AllocIdle idle;
-        return trim_pass(true);
+        const long long freed = trim_pass(true);
+        // a threshold is for callers whose other handles go on (the window
+        // managers); without one the memory is wanted elsewhere
+        if (min_bytes <= 0) pool_release();
+        return freed;
     }
     // the bytes the term-sized buffers hold; released when `release`
     long long trim_pass(bool release)

@@ -468,8 +468,9 @@ int mce_reset(mce_handle* h);
  * window managers call it with 1 GiB on every window they reset, so that
  * only the windows that are large at the same time hold large buffers (the
  * reference's terms are reallocated each step, include/cauchy_estimator.hpp)
- * while small windows keep theirs.  Released memory goes back to the
- * library's pool, which keeps at most a 32nd of the device's memory for its
+ * while small windows keep theirs.  With min_bytes 0 the memory goes back to
+ * the device, and with it what the library's pool held unused; else it goes
+ * back to the pool, which keeps at most a 32nd of the device's memory for its
  * handles' next buffers (256 MiB once no handle and no relative system is
  * alive). */
 long long mce_trim_memory(mce_handle* h, long long min_bytes);

@@ -69,3 +69,18 @@ rel.close()
 assert start - free() <= 256, (start, free())
 print("checked")
 """)
+
+
+def test_trimmed_memory_goes_back_to_the_device():
+    """trim_memory() without a threshold is for those who need the memory
+    elsewhere: the device has it while the handle lives."""
+    _run("""
+b = batch(256)
+b.reset()
+before = free()
+released = b.trim_memory() // MB
+assert released > 512, released
+assert free() - before > 0.9 * released, (before, free(), released)
+b.close()
+print("checked")
+""")
