@@ -1900,7 +1900,7 @@ public:
         MCE_CUDA(cudaMemcpyAsync(cpdf2_y.ptr, ys, sizeof(double) * npts, cudaMemcpyHostToDevice, lc.stream));
         MCE_CUDA(cudaMemsetAsync(counters.ptr + 7, 0, sizeof(int), lc.stream));
         const PdfChunks pc = pdf_chunks(n, npts, 2, lc);
-        if ((s = cpdf_part.ensure((size_t)npts * pc.nch))) return s;
+        if ((s = cpdf_part.ensure(pc.part_size(npts)))) return s;
         cpdf2d_points(cpdf2_tt[e]->ptr, n, MC, cpdf2_x.ptr, cpdf2_y.ptr, npts, est[e].fz[0], pc, cpdf_part.ptr,
                       cpdf2_z.ptr, counters.ptr + 7, lc);
         int bad = 0;
@@ -2115,7 +2115,7 @@ public:
         if ((s = cpdf_y.ensure(npts))) return s;
         MCE_CUDA(cudaMemcpyAsync(cpdf_x.ptr, xs, sizeof(double) * npts, cudaMemcpyHostToDevice, lc.stream));
         const PdfChunks pc = pdf_chunks(n, npts, 1, lc);
-        if ((s = cpdf_part.ensure((size_t)npts * pc.nch))) return s;
+        if ((s = cpdf_part.ensure(pc.part_size(npts)))) return s;
         cpdf1d_points(cpdf_tt[e]->ptr, n, cpdf_x.ptr, npts, exact, est[e].fz[0], pc, cpdf_part.ptr, cpdf_y.ptr, lc);
         MCE_CUDA(cudaMemcpyAsync(ys, cpdf_y.ptr, sizeof(double) * npts, cudaMemcpyDeviceToHost, lc.stream));
         MCE_CUDA(cudaStreamSynchronize(lc.stream));
@@ -2574,7 +2574,7 @@ int rel2d_grid(mce_rel2d* r, double xlow, double xhigh, double dx, double ylow, 
     if ((s = r->xs.ensure(npts))) return s;
     if ((s = r->ys.ensure(npts))) return s;
     if ((s = r->zs.ensure(npts))) return s;
-    if ((s = r->part.ensure((size_t)pc.nch * npts))) return s;
+    if ((s = r->part.ensure(pc.part_size(npts)))) return s;
     if ((s = r->bad.ensure(1))) return s;
     cudaStream_t st = r->stream;
     MCE_CUDA(cudaMemcpyAsync(r->xs.ptr, x, sizeof(double) * npts, cudaMemcpyHostToDevice, st));

@@ -4021,6 +4021,8 @@ void Kernels<D>::rel2d_pairs(const Rel2DArgs& a, const LaunchCfg& c)
 #if MCE_COMMON_UNIT
 // The pdf grids: a thread per (point, chunk of terms), the chunk summed in
 // order into part[chunk * npts + point]; then a warp per point adds its chunks.
+// (Points enough to fill the chip in one chunk each have their sum written
+// where the value goes and scaled there.)
 // A thread per point alone left the chip idle (801 points: 13 blocks of 64
 // threads, each walking 3,324 terms at the latency of a dependent addition):
 // that curve went from 2,726 to 89 us a call, 101 x 83 points of a surface of
@@ -4156,6 +4158,15 @@ __global__ void k_pdf_finish(const double* part, int nch, int npts, int first, d
     if (lane == 0) out[q] = (q < first ? fx * scale0 : scale1 * fx * scale2 * scale2) / fz;
 }
 
+// The same for points of a single chunk, in place: a thread per point.
+__global__ void k_pdf_scale(int npts, int first, double scale0, double scale1, double scale2, double fz, double* out)
+{
+    const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= npts) return;
+    const double fx = out[q];
+    out[q] = (q < first ? fx * scale0 : scale1 * fx * scale2 * scale2) / fz;
+}
+
 // Chunks per point: about `waves` waves of 2,048 threads an SM, at least 8
 // terms a chunk.
 PdfChunks pdf_chunks(long long n, int npts, int waves, const LaunchCfg& c)
@@ -4172,26 +4183,36 @@ PdfChunks pdf_chunks(long long n, int npts, int waves, const LaunchCfg& c)
 
 static inline unsigned pdf_blocks(long long threads) { return (unsigned)((threads + 127) / 128); }
 
+// The points' values from their chunks' sums; a single chunk's are in out.
+static void pdf_finish(const PdfChunks& k, const double* part, int npts, int first, double scale0, double scale1,
+                       double scale2, double fz, double* out, const LaunchCfg& c)
+{
+    ++g_launches;
+    if (k.nch == 1)
+        k_pdf_scale<<<pdf_blocks(npts), 128, 0, c.stream>>>(npts, first, scale0, scale1, scale2, fz, out);
+    else
+        k_pdf_finish<<<pdf_blocks((long long)npts * 32), 128, 0, c.stream>>>(part, k.nch, npts, first, scale0, scale1,
+                                                                            scale2, fz, out);
+}
+
 void cpdf1d_points(const double* tt, long long n, const double* xs, int npts, int exact, double fz,
                    const PdfChunks& k, double* part, double* ys, const LaunchCfg& c)
 {
     if (npts <= 0) return;
-    g_launches += 2;
+    ++g_launches;
     k_cpdf1d_points<<<pdf_blocks((long long)npts * k.nch), 128, 0, c.stream>>>(tt, n, xs, npts, exact, k.chunk, k.nch,
-                                                                              part);
-    k_pdf_finish<<<pdf_blocks((long long)npts * 32), 128, 0, c.stream>>>(part, k.nch, npts, exact, kTwoPiInv, 1.0, 1.0,
-                                                                        fz, ys);
+                                                                              k.nch == 1 ? ys : part);
+    pdf_finish(k, part, npts, exact, kTwoPiInv, 1.0, 1.0, fz, ys, c);
 }
 
 void cpdf2d_points(const double* tt, long long n, int MC, const double* xs, const double* ys, int npts, double fz,
                    const PdfChunks& k, double* part, double* zs, int* bad, const LaunchCfg& c)
 {
     if (npts <= 0) return;
-    g_launches += 2;
+    ++g_launches;
     k_cpdf2d_points<<<pdf_blocks((long long)npts * k.nch), 128, 0, c.stream>>>(
-        tt, nullptr, n, cpdf2d_stride(MC), 1, xs, ys, npts, k.chunk, k.nch, part, bad);
-    k_pdf_finish<<<pdf_blocks((long long)npts * 32), 128, 0, c.stream>>>(part, k.nch, npts, 0, 0.0, 2.0, kTwoPiInv, fz,
-                                                                        zs);
+        tt, nullptr, n, cpdf2d_stride(MC), 1, xs, ys, npts, k.chunk, k.nch, k.nch == 1 ? zs : part, bad);
+    pdf_finish(k, part, npts, 0, 0.0, 2.0, kTwoPiInv, fz, zs, c);
 }
 
 // Relative 2-D pdf (eval_marg2d_relative_and_transformed_cpdf,
@@ -4202,11 +4223,10 @@ void rel2d_points(const double* tt, const long long* kidx, long long nk, int CC,
                   const LaunchCfg& c)
 {
     if (npts <= 0) return;
-    g_launches += 2;
+    ++g_launches;
     k_cpdf2d_points<<<pdf_blocks((long long)npts * k.nch), 128, 0, c.stream>>>(
-        tt, kidx, nk, rel2d_stride(CC), 1 + full, xs, ys, npts, k.chunk, k.nch, part, bad);
-    k_pdf_finish<<<pdf_blocks((long long)npts * 32), 128, 0, c.stream>>>(part, k.nch, npts, 0, 0.0, (double)(2 - full),
-                                                                        kTwoPiInv, nf, zs);
+        tt, kidx, nk, rel2d_stride(CC), 1 + full, xs, ys, npts, k.chunk, k.nch, k.nch == 1 ? zs : part, bad);
+    pdf_finish(k, part, npts, 0, 0.0, (double)(2 - full), kTwoPiInv, nf, zs, c);
 }
 
 // kidx[kpos[j]] = j for every kept pair j (kpos: exclusive scan of keep)

@@ -291,10 +291,11 @@ struct Kernels {
 void group_count(const int* status, const int* owner, const int* m, long long nR, int D, int* gcnt, int* is_root,
                  int* cap, int* alive, const LaunchCfg& c);
 // The pdf grids' split of n terms over npts points: nch chunks of `chunk`
-// terms per point, their sums in part[nch * npts].
+// terms per point, their sums in part[part_size(npts)].
 struct PdfChunks {
     long long chunk = 1;
     int nch = 1;
+    size_t part_size(int npts) const { return nch > 1 ? (size_t)nch * npts : 0; }
 };
 PdfChunks pdf_chunks(long long n, int npts, int waves, const LaunchCfg& c);
 // doubles per term record of the marginal 2-D pdf

@@ -84,3 +84,28 @@ assert free() - before > 0.9 * released, (before, free(), released)
 b.close()
 print("checked")
 """)
+
+
+def test_a_grid_in_one_chunk_takes_no_partial_sums():
+    """A pdf surface of so many points that each sums its terms in one go
+    needs the points and the values, 24 bytes a point, and no more; the values
+    are those of the same points in a small grid."""
+    _run("""
+e = estimator(W.two_state_lti, 1)
+nu = np.array([0.7, 1.3])
+e.cpdf_2d_grid(0, 0, 1, (-1.0, 1.0, 0.25), (-1.0, 1.0, 0.25), nu)
+start = free()
+X, Y, Z = e.cpdf_2d_grid(0, 0, 1, (-1.0, 1.0, 2.0 ** -12), (-1.0, 1.0, 2.0 ** -10), nu)
+took = (start - free()) * MB
+assert len(X) == 8193 * 2049
+assert took <= 26 * len(X) + 64 * MB, took / len(X)
+x, y, z = e.cpdf_2d_grid(0, 0, 1, (-1.0, 1.0, 0.25), (-1.0, 1.0, 0.25), nu)
+at = np.searchsorted(Y.reshape(2049, 8193)[:, 0], y) * 8193 + np.searchsorted(X[:8193], x)
+assert np.array_equal(X[at], x) and np.array_equal(Y[at], y)
+assert np.allclose(Z[at], z, rtol=1e-12, atol=0.0)
+xs, ys = e.cpdf_1d_grid(0, 0, -1.0, 1.0, 2.0 ** -20, nu)
+xt, yt = e.cpdf_1d_grid(0, 0, -1.0, 1.0, 0.125, nu)
+at = np.searchsorted(xs, xt)
+assert np.array_equal(xs[at], xt) and np.allclose(ys[at], yt, rtol=1e-9, atol=0.0)
+print("checked")
+""")
