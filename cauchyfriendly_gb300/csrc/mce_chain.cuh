@@ -117,6 +117,7 @@ constexpr int kChainTile = kChainThreads * kChainRun; // rows a tile
 constexpr int kChainPitch = kChainRun + 2;            // doubles between the threads' runs in shared memory
 constexpr int kChainStages = 3;
 constexpr int kChainRounds = 12;
+static_assert(kChainRun % 2 == 0 && kChainPitch % 2 == 0, "a thread's run starts on 16 bytes");
 
 struct ChainMap {  // x -> c + RN_u(x + b), u a power of two (1: exact)
     long long b, c, u;
@@ -142,7 +143,8 @@ __device__ inline long long chain_units(double x, int q)
     return (int)hi < 0 ? -r : r;
 }
 
-struct ChainSmem {
+// (16-byte copies land in v, and are read from it)
+struct alignas(16) ChainSmem {
     double v[kChainStages][kChainThreads * kChainPitch];
     double h[kChainThreads / 32], p[kChainThreads / 32], s;
     ChainMap m[kChainThreads / 32];
