@@ -266,3 +266,37 @@ def test_gpu_pdf_grids_do_not_depend_on_how_the_terms_are_split(updates, nx, ny)
     assert len(X) == nx * ny and np.array_equal(X, Xo.reshape(-1)) and np.array_equal(Y, Yo.reshape(-1))
     assert G.relerr(Z, Zo.reshape(-1)) <= G.REL_TOL
     est.close()
+
+
+@pytest.mark.parametrize("d,pncc,updates,rows", [(2, 6, 2, 8), (2, 7, 2, 9), (2, 7, 3, 16), (3, 5, 2, 8), (3, 6, 2, 9),
+                                                 (3, 7, 2, 10), (3, 6, 3, 15), (4, 4, 2, 8), (4, 5, 2, 9),
+                                                 (4, 6, 2, 10), (4, 6, 3, 16)])
+def test_gpu_nd_pdf_at_the_row_limits_of_its_paths(d, pncc, updates, rows):
+    """Terms of up to 8, 9 and 10 rows (cells by a thread up to parents of 8,
+    rows of a child in 8 or 15 places) and of 15 and 16, the most: the pdf of
+    the full state and of the first states alone, against the oracle lowering
+    every child apart."""
+    _, CE, _ = _need_gpu()
+    from cauchyfriendly_gb300 import workloads as W
+    prob = W.many_gamma(d, pncc, updates + 1, seed=3)
+    rp, bp = oracle.draw_reference_constants(23, d, oracle.max_shape_of(prob))
+    est = _stepped_gpu(CE, prob, rp, bp, updates)
+    orc = oracle.Oracle(prob, rp, bp)
+    for k in range(updates):
+        orc.step(k)
+    assert np.nonzero(est.terms_per_shape())[0].max() == rows
+    mu = orc.moments()["mean"].real
+    X = mu + np.array([0.0, 0.1, -0.3])[:, None] * np.ones(d)
+    got = est.cpdf_nd(X)
+    want = np.array([orc.cpdf_nd(x, reduce=False) for x in X])
+    close = lambda a, b: np.max(np.abs(a - b) / np.maximum(np.abs(b), 1e-3 * np.abs(b).max()))
+    assert close(got, want) <= G.REL_TOL, close(got, want)
+    for keep in range(1, d):
+        nu = np.cos(1.0 + 2.3 * np.arange(d - keep))
+        idx = list(range(keep))
+        got = est.cpdf_marginal(X[:, :keep], idx, nu)
+        want = np.array([orc.cpdf_marginal(x[:keep], idx, nu, reduce=False) for x in X])
+        assert close(got, want) <= G.REL_TOL, (keep, close(got, want))
+    assert est.device_errors() == 0
+    est.close()
+    orc.close()

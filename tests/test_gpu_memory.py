@@ -1,9 +1,13 @@
-"""Device memory the library keeps between uses, looked at from a process of
+"""Device memory the library keeps between uses: what it hands back, what is
+there for its own other buffers when the device is full, and handles that
+grow and go on several threads at once.  Memory is looked at from a process of
 its own, in which nothing else holds any."""
 import os
 import subprocess
 import sys
+import threading
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -71,6 +75,54 @@ print("checked")
 """)
 
 
+@pytest.mark.parametrize("what", ["points", "gradient"])
+def test_buffers_outside_the_pool_on_a_full_device(what):
+    """The pool holds gigabytes that no handle uses and the rest of the device
+    is taken: the pdf at points and the gradient, whose buffers are not the
+    pool's, find their memory there."""
+    _run("""
+what = %r
+x = rng.standard_normal((16, 4))
+q = W.four_state_lti(seed=0, steps=7)
+n = 24
+
+def call():
+    if what == "points":
+        return small.cpdf_nd(x)
+    c = np.random.Generator(np.random.PCG64(2))
+    runs = AdjointBatch(4, 1, 1, [7] * n, np.stack([q["A0"]] * n), np.stack([q["p0"]] * n), np.stack([q["b0"]] * n),
+                        1.0 + c.uniform(size=(n, 4)), c.uniform(-1.0, 1.0, (n, 10)))
+    fz = runs.forward([q["msmts"].reshape(-1)] * n, *[q[k] for k in ("Phi", "Gamma", "beta", "H", "gamma")])
+    g = runs.backward([loglik_weights(f) for f in fz])
+    out = np.concatenate([np.concatenate(fz)] + [r[k].reshape(-1) for r in g for k in sorted(r)])
+    runs.close()
+    return out
+
+small = estimator(W.four_state_lti, 5)
+other = estimator(W.four_state_lti, 5)
+want = call()
+small.close()
+small = estimator(W.four_state_lti, 5)
+want = call()
+small.close()
+rng = np.random.Generator(np.random.PCG64(1))
+small = estimator(W.four_state_lti, 5)
+before = free()
+want = call()
+small.close()
+rng = np.random.Generator(np.random.PCG64(1))
+small = estimator(W.four_state_lti, 5)
+held = free()
+big = batch(1024)
+big.close()
+assert held - free() > 3500, (held, free())  # more than the call takes
+filler = torch.empty((free() - 256) * MB, dtype=torch.uint8, device="cuda")
+got = call()
+assert np.allclose(got, want, rtol=1e-9, atol=1e-12 * np.abs(want).max())
+print("checked")
+""" % what)
+
+
 def test_trimmed_memory_goes_back_to_the_device():
     """trim_memory() without a threshold is for those who need the memory
     elsewhere: the device has it while the handle lives."""
@@ -109,3 +161,53 @@ at = np.searchsorted(xs, xt)
 assert np.array_equal(xs[at], xt) and np.allclose(ys[at], yt, rtol=1e-9, atol=0.0)
 print("checked")
 """)
+
+
+def test_handles_growing_and_going_on_several_threads():
+    """Four threads make, step, trim and destroy batches of their own sizes,
+    whose buffers pass from one to another through the pool: the results are
+    those of one thread."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from cauchyfriendly_gb300 import BatchedCauchyEstimator
+    from cauchyfriendly_gb300 import workloads as W
+
+    def run(n, seed):
+        probs = W.batched_three_state(n, seed=seed, steps_lo=4, steps_hi=7)
+        rng = np.random.Generator(np.random.PCG64(seed))
+        s = lambda k: np.stack([q[k] for q in probs])
+        z = np.zeros((n, 7, 1))
+        for i, q in enumerate(probs):
+            z[i, :q["steps"]] = q["msmts"]
+        b = BatchedCauchyEstimator(s("A0"), s("p0"), s("b0"), np.array([q["steps"] for q in probs], np.int32), 3, 0, 1,
+                                   1, 1.0 + rng.uniform(size=(n, 3)), rng.uniform(-1.0, 1.0, (n, 9)))
+        out = []
+        for _ in range(2):
+            out.append(b.run(z, *[s(k) for k in ("Phi", "Gamma", "beta", "H", "gamma")], shared_model=False))
+            b.reset()
+            b.trim_memory(1 << 20)
+        b.close()
+        return out
+
+    jobs = [(n, 10 * t + r) for t in range(4) for r, n in enumerate((17, 160, 41, 300))]
+    want = {j: run(*j) for j in jobs}
+    got, failed = {}, []
+
+    def work(t):
+        try:
+            for j in jobs[4 * t: 4 * t + 4]:
+                got[j] = run(*j)
+        except Exception as e:  # pragma: no cover
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    for j in jobs:
+        for a, b in zip(got[j], want[j]):
+            for k in a:
+                assert np.array_equal(a[k], b[k], equal_nan=True), (j, k)

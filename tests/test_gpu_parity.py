@@ -489,3 +489,43 @@ def test_flat_groups_of_more_than_sixteen_rows():
     assert np.array_equal(a["shape"], b["shape"]) and np.array_equal(a["cells"], b["cells"])
     assert np.array_equal(a["keys"], b["keys"])
     assert G.relerr(a["g"], b["g"]) <= G.REL_TOL, G.relerr(a["g"], b["g"])
+
+
+@pytest.mark.parametrize("states,updates,alone", [(3, 8, 5), (4, 6, 3)])
+def test_long_buckets_of_the_term_reduction(states, updates, alone):
+    """Measurements of zero leave every term at b = 0, so that all terms of a
+    shape share a bucket.  Estimators stepped together make steps of more than
+    2^14 records, whose long buckets go to a list of their own; each steps as
+    it does alone, where no such list is kept, bit for bit."""
+    CE, BCE = _gpu()
+    from cauchyfriendly_gb300 import workloads as W
+    prob = (W.three_state_lti if states == 3 else W.four_state_lti)(seed=0, steps=updates + 1)
+    n = 2 * alone
+    ms = oracle.max_shape_of(prob)
+    rp, bp = oracle.draw_reference_constants(7, states, ms)
+    z = np.zeros((n, updates))
+    z[1::2] = prob["msmts"][:updates, 0]  # every other one with measurements
+    tile = lambda a: np.broadcast_to(a, (n,) + a.shape)
+    bat = BCE(tile(prob["A0"]), tile(prob["p0"]), tile(prob["b0"]), [updates + 1] * n, states, 0, 1, 1, tile(rp),
+              tile(bp))
+    ones = [CE(prob["A0"], prob["p0"], prob["b0"], updates + 1, states, 0, 1, 1, root_point=rp, b_pert=bp)
+            for _ in range(2)]
+    model = (prob["Phi"], prob["Gamma"], prob["beta"], prob["H"][0], prob["gamma"][0])
+    for k in range(updates):
+        bat.step(z[:, k], model[0], model[1], model[2], tile(model[3]), np.full(n, model[4]), shared_model=True)
+        for e, a in enumerate(ones):
+            a.step(z[e, k], *model)
+        for e in (0, 1, n - 2, n - 1):
+            a = ones[e % 2]
+            assert bat.num_terms(e) == a.num_terms(), (k, e)
+            assert np.array_equal(bat.terms_per_shape(e), a.terms_per_shape())
+            mb, ma = bat.moments(e), a.moments()
+            for key in ("raw_fz", "raw_mean", "raw_cov"):
+                assert G.bitwise_equal(np.atleast_1d(mb[key]), np.atleast_1d(ma[key])), (k, e, key)
+    for e in (0, 1, n - 2, n - 1):
+        tb, ta = bat.dump_terms(e), ones[e % 2].dump_terms(0)
+        for key in ta:
+            assert G.bitwise_equal(tb[key], ta[key]), (e, key)
+    for a in ones:
+        a.close()
+    bat.close()
