@@ -597,7 +597,7 @@ def run_rel2d(args):
     peak, peak_kind = measured_peaks()
     ms_pairs, ms_grid = tot["pairs"] / args.steps, tot["grid"] / args.steps
     top = "grid" if ms_grid >= ms_pairs else "pairs"
-    roofline = {"bound": "hbm", "kernel": "k_rel2d_points" if top == "grid" else "k_rel2d_pairs",
+    roofline = {"bound": "hbm", "kernel": "k_cpdf2d_points" if top == "grid" else "k_rel2d_pairs",
                 "achieved": (pair_bytes / (ms_pairs / 1e3) if top == "pairs" else
                              8.0 * kept * (6 * mean_cells + 5) / (ms_grid / 1e3)) / 1e9,
                 "peak": peak, "unit": "GB/s", "peak_source": peak_kind, "traffic": None,

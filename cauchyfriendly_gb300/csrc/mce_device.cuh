@@ -255,8 +255,11 @@ __device__ inline int orientation_mask(const double* Ai, const double* Aj, int m
 
 // A product of the unrolled elimination and solves: on the integer pipe up to
 // D = 3, whose code still fits the instruction cache (k_build_B_vertices<3> in
-// the 331-estimator batch's last update 599 -> 483 us; with D = 5 the same
-// products took a 5-state window's 71 ms to 94).
+// the 331-estimator batch's last update 599 -> 483 us).  Above, the same
+// products and the unrolled condition loop cost more than they save: D = 4,
+// eight updates of one estimator 260 us without and 285 with them, a pass of
+// its sliding windows 1.15 ms and 1.55; D = 5, a pass of 5-state windows 71 ms
+// and 94.
 template <int D>
 __device__ inline double lu_mul(double a, double b)
 {

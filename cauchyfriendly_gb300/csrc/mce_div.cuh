@@ -26,7 +26,7 @@
 // the 5-state relative system's pairs and 13 x 13 grid from 1,177 to 728 ms,
 // 256 points of the 4-state joint pdf from 322 to 211 ms.
 //
-// Operands outside [2^-255, 2^256) take the ordinary division (zeros over an
+// Operands outside [2^-255, 2^257) take the ordinary division (zeros over an
 // operand inside give the signed zero at once), so no result of the long
 // division is subnormal or overflows.
 #pragma once
@@ -168,7 +168,7 @@ MCE_HD inline double divide(double a, double b) { return divide(a, div_by(b)); }
 // (one of each in turn: 10.3 cycles an operation).  How many is each kernel's
 // balance between the two pipes, divisions included.  Zeros, which structured
 // models are full of, are answered at once; other operands outside
-// [2^-255, 2^256) take the FP64 pipe (a call, so that the compiler does not run
+// [2^-255, 2^257) take the FP64 pipe (a call, so that the compiler does not run
 // both).
 #ifdef __CUDACC__
 static __device__ __noinline__ double mul_slow(double a, double b) { return a * b; }

@@ -36,7 +36,7 @@ namespace mce {
 
 extern thread_local std::string g_last_error;
 // Set by mce_batch_step_noalloc for the duration of its step: a DevBuf that
-// would have to grow fails with MCE_ERR_NOMEM instead of calling cudaMalloc.
+// would have to grow fails with MCE_ERR_NOMEM instead of allocating.
 extern thread_local bool g_device_alloc_forbidden;
 #if MCE_ONLY_DIM <= 0
 thread_local std::string g_last_error;
@@ -65,6 +65,10 @@ static void set_error(const std::string& s) { g_last_error = s; }
 // and allocated in the order of the handle's stream, on which all of a step's
 // work is queued or joined; elsewhere an allocation is complete, and a freed
 // buffer's work done, before the call returns, as with cudaMalloc and cudaFree.
+// A cudaMalloc of this process (the point-wise pdf's and the adjoint's buffers,
+// another library's) that finds the device full gets what the pool holds
+// unused: the driver frees it (254 MB free beside 5.5 GB in the pool: 1.2 GB
+// allocated).
 constexpr size_t kPoolKeepIdle = 256u << 20;
 extern thread_local cudaStream_t t_alloc_stream;  // of the step this thread is in, or null
 extern thread_local bool t_alloc_idle;            // the buffers being freed have no work left
@@ -205,7 +209,8 @@ struct DevBuf {
         const cudaError_t e = dev_malloc(&q, want * sizeof(T));
         if (e != cudaSuccess) {
             cudaGetLastError();
-            set_error("cudaMalloc of " + std::to_string(want * sizeof(T)) + " bytes failed: " + cudaGetErrorString(e));
+            set_error("device allocation of " + std::to_string(want * sizeof(T)) + " bytes failed: " +
+                      cudaGetErrorString(e));
             return MCE_ERR_NOMEM;
         }
         ptr = static_cast<T*>(q);

@@ -7,7 +7,8 @@
 // allocation failure mid-run as unacceptable), and any caller for which the
 // device-wide synchronisation of cudaMalloc/cudaFree would stall work on
 // other streams.  mce_batch_step grows the handle's buffers, and its g-table
-// kernel's per-warp scratch, with cudaMalloc whenever a step needs more room.
+// kernel's per-warp scratch, from the library's stream-ordered pool whenever a
+// step needs more room, and the pool grows from the device.
 //
 // This entry point runs the same step with two differences:
 //  * the g-table kernel (k_gtable) takes its per-warp scratch from the
@@ -15,7 +16,7 @@
 //    as many warps as the array has slots for; the warps stride over the
 //    roots, so the tables are the same;
 //  * no device buffer of the handle may grow: one that would have to fails
-//    the call with MCE_ERR_NOMEM instead of calling cudaMalloc.
+//    the call with MCE_ERR_NOMEM instead of allocating.
 // It calls no cudaMalloc, cudaFree or other allocating routine.
 //
 // The array is shared by every call in the process on a device and keeps the
