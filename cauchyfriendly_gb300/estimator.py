@@ -160,8 +160,9 @@ class BatchedCauchyEstimator:
 
     def trim_memory(self, min_bytes=0):
         """Frees the device buffers that grow with the term count (between a
-        reset and the next step) when they hold at least min_bytes; returns
-        the bytes released."""
+        reset and the next step) when they hold at least min_bytes, for other
+        handles or, without a threshold, back to the device; returns the
+        bytes released."""
         return _lib.check(self._lib.mce_trim_memory(self._h, int(min_bytes)), "mce_trim_memory")
 
     def reinitialize_start_statistics(self, A0, p0, b0, e=0):
